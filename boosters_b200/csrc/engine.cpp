@@ -3265,12 +3265,12 @@ void forest_predict_rows(const DeviceForest& f, const float* x, uint64_t n, uint
     }
     const size_t need = predict_heap_scratch(f.heap, (uint32_t)F, n);
     if (scratch && scratch_bytes >= need) {
-        launch_predict_heap(f.heap, x, n, (uint32_t)F, out, scratch, st);
+        launch_predict_heap(f.heap, x, n, (uint32_t)F, 0, out, scratch, st);
         return;
     }
     void* tmp = nullptr;
     BST_CK(cudaMallocFromPoolAsync(&tmp, std::max<size_t>(need, 16), scratch_pool(), st));
-    launch_predict_heap(f.heap, x, n, (uint32_t)F, out, tmp, st);
+    launch_predict_heap(f.heap, x, n, (uint32_t)F, 0, out, tmp, st);
     BST_CK(cudaFreeAsync(tmp, st));
 }
 

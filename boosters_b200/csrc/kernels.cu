@@ -4416,15 +4416,10 @@ constexpr uint32_t PREDICT_TREE_BYTES = HEAP_NODES * 4u;
 constexpr uint32_t PREDICT_RING = 2u * PREDICT_CHUNK * PREDICT_TREE_BYTES;
 constexpr uint32_t PREDICT_MAX_ROWS = PREDICT_TILE_MAX;
 constexpr uint32_t PREDICT_MIN_ROWS = 128;
-constexpr uint32_t PREDICT_SPL_MAX_F = 256;  // splitter table in shared memory up to this many features
 constexpr uint32_t BIN_NAN = 0xFFFFu;
 constexpr uint32_t BIN_THREADS = 256;         // binning pass: 8 warps per block
-constexpr uint32_t BIN_F = 8;                 // features staged per step of the binning pass
-constexpr uint32_t BIN_XS_LD = BIN_F + 1;     // floats per staged row: odd stride
-
-__host__ __device__ inline uint32_t predict_spl_floats(uint32_t NF) {
-    return NF <= PREDICT_SPL_MAX_F ? NF * HEAP_SPLITTERS : 0u;
-}
+constexpr uint32_t BIN_F = 8;                 // features per block of the binning pass at most
+constexpr uint32_t BIN_TAB = 256;             // staged thresholds per feature: a search tree of 8 levels
 
 // Launch shape of the traversal: R rows per tile, the trees of each chunk
 // split over S thread groups of R threads (S > 1 for small batches: each
@@ -4485,11 +4480,21 @@ __device__ __forceinline__ uint32_t heap_bin_block(const float* __restrict__ t, 
     return k + (t[k] <= v ? 1u : 0u);
 }
 
-// Binning pass: one warp bins 32 * RPL rows (lane l: rows l + 32 i), all
-// features, PREDICT_BIN_F at a time staged through shared memory (coalesced
-// loads), into the tile layout; the RPL rows of a lane fill one 32-bit word
-// per column.
-template <typename BinT>
+// Binning pass. A block takes up to FC features and stages their thresholds
+// in shared memory in heap order (level l of the search tree at entries
+// 2^l .. 2^(l+1) - 1, so the lanes of a step read one contiguous run of
+// words: no bank conflict up to 32 entries), then its warps bin 32 * RPL rows
+// at a time (lane l: rows l + 32 i; the RPL rows of a lane fill one 32-bit
+// word per column of the tile layout). FM: x is feature-major [F][n] (lanes
+// read consecutive rows); else sample-major [n][F], staged through shared
+// memory FC features at a time.
+//
+// The pass is bound by the searches' shared-memory wavefronts: one per level
+// and 32 rows for the first six levels, about two for the two levels below.
+// The form before it searched a sorted 16-entry splitter table (bank
+// conflicts: the steps' strides are powers of two) and a 16-entry block in
+// global memory (up to eight cache lines per step).
+template <typename BinT, bool FM>
 __global__ void __launch_bounds__(BIN_THREADS)
 k_bin_rows(HeapForest f, const float* __restrict__ x, uint64_t n, uint32_t F, uint32_t R, uint32_t FC,
            uint32_t* __restrict__ bins_g) {
@@ -4498,90 +4503,157 @@ k_bin_rows(HeapForest f, const float* __restrict__ x, uint64_t n, uint32_t F, ui
     constexpr uint32_t WR = 32u * RPL;  // rows per warp
     constexpr uint32_t BITS = 8u * (uint32_t)sizeof(BinT);
     extern __shared__ __align__(16) float bsm[];
+    __shared__ uint32_t s_lev[BIN_F];  // search levels of each staged feature (0: search in global memory)
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarps = BIN_THREADS / 32u;
     const uint32_t NF = F < f.n_features ? F : f.n_features;
-    const uint32_t spl_n = predict_spl_floats(NF);
-    float* spl = bsm;
-    float* xs = bsm + spl_n + (size_t)warp * WR * BIN_XS_LD;
-    for (uint32_t i = tid; i < spl_n; i += BIN_THREADS) spl[i] = f.spl[i];
+    const uint32_t n_fc = (NF + FC - 1) / FC;
+    const uint32_t fc = blockIdx.x % n_fc;
+    const uint32_t f0 = fc * FC, f1 = f0 + FC < NF ? f0 + FC : NF, nf = f1 - f0;
+    float* tab = bsm;  // [FC][BIN_TAB]
+    const uint32_t xld = FC | 1u;  // floats per staged row: odd stride
+    float* xs = bsm + FC * BIN_TAB + (size_t)warp * WR * xld;
+    if (tid < nf) {
+        const uint32_t o = f.thr_off[f0 + tid], e = f.thr_off[f0 + tid + 1] - o;  // e: padded entries
+        uint32_t lev = 0;
+        if (!(f.feat_info[f0 + tid] >> 7)) {
+            if (e <= 240u || (e == 256u && f.thr[o + 255] != f.thr[o + 255])) {  // at most 255 thresholds
+                lev = 1;
+                while (lev < 8u && (1u << lev) - 1u < e) ++lev;
+            }
+        }
+        s_lev[tid] = lev;
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < nf * BIN_TAB; i += BIN_THREADS) {
+        const uint32_t j = i / BIN_TAB, k = i % BIN_TAB, lev = s_lev[j];
+        float v = NAN;  // never <= x
+        if (!lev) {  // searched in global memory: the splitters
+            if (k < HEAP_SPLITTERS) v = f.spl[(size_t)(f0 + j) * HEAP_SPLITTERS + k];
+        } else if (k && k < (1u << lev)) {
+            const uint32_t l = 31u - (uint32_t)__clz(k);
+            const uint32_t at = (2u * (k - (1u << l)) + 1u) * (1u << (lev - 1u - l)) - 1u;  // in sorted order
+            const uint32_t o = f.thr_off[f0 + j];
+            if (at < f.thr_off[f0 + j + 1] - o) v = f.thr[o + at];
+        }
+        tab[i] = v;
+    }
     __syncthreads();
     const uint32_t col_words = R * (uint32_t)sizeof(BinT) / 4u;
     const uint64_t n_groups = (n + WR - 1) / WR;
-    const uint32_t n_fc = (NF + FC - 1) / FC;  // feature chunks: more warps for a small batch
-    const uint64_t items = n_groups * n_fc;
-    for (uint64_t it = (uint64_t)blockIdx.x * nwarps + warp; it < items; it += (uint64_t)gridDim.x * nwarps) {
-        const uint64_t gi = it / n_fc;
-        const uint32_t f0 = (uint32_t)(it - gi * n_fc) * FC, f1 = f0 + FC < NF ? f0 + FC : NF;
+    const uint64_t rb = blockIdx.x / n_fc, n_rb = gridDim.x / n_fc;  // the grid is a multiple of n_fc
+    for (uint64_t gi = rb * nwarps + warp; gi < n_groups; gi += n_rb * nwarps) {
         const uint64_t row0 = gi * WR;
         const uint64_t tile = row0 / R;
         const uint32_t rg0 = (uint32_t)(row0 - tile * R);  // a multiple of WR
         const uint32_t nr = (uint32_t)(n - row0 < WR ? n - row0 : WR);
         uint32_t* tw = bins_g + (size_t)tile * f.n_cols * col_words + (rg0 / WR) * 32u + lane;
-        for (uint32_t fg = f0; fg < f1; fg += BIN_F) {
-            const uint32_t fj = fg + lane % BIN_F;
+        if constexpr (!FM) {
+            if (nf == BIN_F) {
 #pragma unroll 8
-            for (uint32_t k = 0; k < WR * BIN_F / 32u; ++k) {
-                const uint32_t row = lane / BIN_F + k * (32u / BIN_F);
-                xs[row * BIN_XS_LD + lane % BIN_F] = row < nr && fj < f1 ? x[(row0 + row) * F + fj] : 0.0f;
+                for (uint32_t k = 0; k < WR * BIN_F / 32u; ++k) {
+                    const uint32_t row = lane / BIN_F + k * (32u / BIN_F);
+                    xs[row * xld + lane % BIN_F] = row < nr ? x[(row0 + row) * F + f0 + lane % BIN_F] : 0.0f;
+                }
+            } else {
+                for (uint32_t k = lane; k < WR * nf; k += 32u) {
+                    const uint32_t row = k / nf, j = k % nf;
+                    xs[row * xld + j] = row < nr ? x[(row0 + row) * F + f0 + j] : 0.0f;
+                }
             }
             __syncwarp();
-            const uint32_t nf = f1 - fg < BIN_F ? f1 - fg : BIN_F;
-            for (uint32_t j = 0; j < nf; ++j) {
-                const uint32_t ft = fg + j;  // the same feature in every lane
-                const int32_t c0 = f.feat_col[2 * ft], c1 = f.feat_col[2 * ft + 1];
-                if (c0 < 0 && c1 < 0) continue;
-                const uint32_t info = f.feat_info[ft];
-                const uint32_t lb = info & 31u;
-                const float* sp = spl_n ? spl + ft * HEAP_SPLITTERS : f.spl + (size_t)ft * HEAP_SPLITTERS;
-                const float* t = f.thr + f.thr_off[ft];
-                float v[RPL];
-                uint32_t b[RPL];
+        }
+        for (uint32_t j = 0; j < nf; ++j) {
+            const uint32_t ft = f0 + j;  // the same feature in every lane
+            const int32_t c0 = f.feat_col[2 * ft], c1 = f.feat_col[2 * ft + 1];
+            if (c0 < 0 && c1 < 0) continue;
+            const uint32_t info = f.feat_info[ft];
+            float v[RPL];
+            uint32_t b[RPL];
 #pragma unroll
-                for (uint32_t i = 0; i < RPL; ++i) {
-                    v[i] = xs[(lane + 32u * i) * BIN_XS_LD + j];
-                    b[i] = 0;
-                }
-                if (!(info >> 7)) {
+            for (uint32_t i = 0; i < RPL; ++i) {
+                if constexpr (FM)
+                    v[i] = lane + 32u * i < nr ? x[(uint64_t)ft * n + row0 + lane + 32u * i] : 0.0f;
+                else
+                    v[i] = xs[(lane + 32u * i) * xld + j];
+                b[i] = 0;
+            }
+            if (!(info >> 7)) {
+                const uint32_t lev = s_lev[j];
+                if (lev) {  // b: heap position, then the number of thresholds <= v
+                    const float* t = tab + j * BIN_TAB;
+#pragma unroll
+                    for (uint32_t i = 0; i < RPL; ++i) b[i] = 1u;
+                    if (lev == 8u) {  // 128 thresholds or more
+#pragma unroll
+                        for (uint32_t s = 0; s < 8u; ++s) {
+#pragma unroll
+                            for (uint32_t i = 0; i < RPL; ++i) b[i] = 2u * b[i] + (t[b[i]] <= v[i] ? 1u : 0u);
+                        }
+                    } else {
+                        for (uint32_t s = 0; s < lev; ++s) {
+#pragma unroll
+                            for (uint32_t i = 0; i < RPL; ++i) b[i] = 2u * b[i] + (t[b[i]] <= v[i] ? 1u : 0u);
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t i = 0; i < RPL; ++i) b[i] -= 1u << lev;
+                } else {
+                    const uint32_t lb = info & 31u;
+                    const float* sp = tab + j * BIN_TAB;
+                    const float* t = f.thr + f.thr_off[ft];
 #pragma unroll
                     for (uint32_t s = HEAP_SPLITTERS / 2; s >= 1; s >>= 1) {
 #pragma unroll
                         for (uint32_t i = 0; i < RPL; ++i) b[i] += sp[b[i] + s - 1] <= v[i] ? s : 0u;
                     }
-                    if (lb == 4) {  // 16-entry blocks: fixed steps, the rows interleaved
 #pragma unroll
-                        for (uint32_t i = 0; i < RPL; ++i) b[i] <<= 4;
-#pragma unroll
-                        for (uint32_t s = 8; s >= 1; s >>= 1) {
-#pragma unroll
-                            for (uint32_t i = 0; i < RPL; ++i) b[i] += t[b[i] + s - 1] <= v[i] ? s : 0u;
-                        }
-#pragma unroll
-                        for (uint32_t i = 0; i < RPL; ++i) b[i] += t[b[i]] <= v[i] ? 1u : 0u;
-                    } else {
-#pragma unroll
-                        for (uint32_t i = 0; i < RPL; ++i) b[i] = heap_bin_block(t, lb, b[i], v[i]);
-                    }
+                    for (uint32_t i = 0; i < RPL; ++i) b[i] = heap_bin_block(t, lb, b[i], v[i]);
                 }
-                uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-                for (uint32_t i = 0; i < RPL; ++i) {
-                    uint32_t bb = b[i];
-                    if (v[i] != v[i]) {
-                        bb = BIN_NAN;
-                    } else if (info >> 7) {
-                        const uint32_t cv = sat_u32(v[i]);
-                        bb = cv < 65534u ? cv : 65534u;
-                    }
-                    const uint32_t mask = (1u << BITS) - 1u;  // NaN: largest bin / 0
-                    w0 |= (bb == BIN_NAN ? mask : bb & mask) << (BITS * i);
-                    w1 |= (bb == BIN_NAN ? 0u : bb & mask) << (BITS * i);
-                }
-                if (c0 >= 0) tw[(size_t)c0 * col_words] = w0;
-                if (c1 >= 0) tw[(size_t)c1 * col_words] = w1;
             }
-            __syncwarp();
+            uint32_t w0 = 0, w1 = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < RPL; ++i) {
+                uint32_t bb = b[i];
+                if (v[i] != v[i]) {
+                    bb = BIN_NAN;
+                } else if (info >> 7) {
+                    const uint32_t cv = sat_u32(v[i]);
+                    bb = cv < 65534u ? cv : 65534u;
+                }
+                const uint32_t mask = (1u << BITS) - 1u;  // NaN: largest bin / 0
+                w0 |= (bb == BIN_NAN ? mask : bb & mask) << (BITS * i);
+                w1 |= (bb == BIN_NAN ? 0u : bb & mask) << (BITS * i);
+            }
+            if (c0 >= 0) tw[(size_t)c0 * col_words] = w0;
+            if (c1 >= 0) tw[(size_t)c1 * col_words] = w1;
         }
+        __syncwarp();  // xs is rewritten for the next rows
     }
+}
+
+// Features per block of the binning pass: the most (8, a sector of a
+// sample-major row) that still gives every SM a block; one per block for the
+// smallest batches, whose time is one block's latency.
+static uint32_t bin_rows_features(uint32_t NF, uint64_t row_blocks) {
+    uint32_t fc = BIN_F;
+    while (fc > 1 && (NF + fc - 1) / fc * row_blocks < sm_count()) fc >>= 1;
+    return fc;
+}
+
+template <typename BinT, bool FM>
+static void launch_bin_rows(const HeapForest& f, const float* x, uint64_t n, uint32_t F, uint32_t R, void* scratch,
+                            cudaStream_t st) {
+    const uint32_t NF = F < f.n_features ? F : f.n_features;
+    const uint32_t wr = 32u * (4u / (uint32_t)sizeof(BinT));
+    const uint64_t groups = (n + wr - 1) / wr;
+    const uint64_t row_blocks = (groups + BIN_THREADS / 32u - 1) / (BIN_THREADS / 32u);
+    const uint32_t FC = bin_rows_features(NF, row_blocks);
+    const uint32_t n_fc = (NF + FC - 1) / FC;
+    // about four resident blocks per SM, each looping over its share of the rows
+    const uint64_t most = (sm_count() * 4u + n_fc - 1) / n_fc;
+    const unsigned grid = n_fc * (unsigned)(row_blocks < most ? row_blocks : most);
+    const size_t smem = (FC * BIN_TAB + (FM ? 0 : (size_t)(BIN_THREADS / 32u) * wr * (FC | 1u))) * sizeof(float);
+    launch_k(k_bin_rows<BinT, FM>, grid, BIN_THREADS, smem, st, f, x, n, F, R, FC, static_cast<uint32_t*>(scratch));
 }
 
 // One split step: from heap position h of tree to its chosen child. cb: this
@@ -4701,32 +4773,18 @@ k_predict_heap(HeapForest f, const unsigned char* __restrict__ bins_g, uint64_t 
     }
 }
 
-void launch_predict_heap(const HeapForest& f, const float* x, uint64_t n, uint32_t F, float* out, void* scratch,
-                         cudaStream_t st) {
+void launch_predict_heap(const HeapForest& f, const float* x, uint64_t n, uint32_t F, int feature_major, float* out,
+                         void* scratch, cudaStream_t st) {
     if (n == 0) return;
     init_kernel_attributes();  // per device: the kernels' shared-memory opt-in
     const HeapPlan p = heap_plan(f, F, n);
-    const uint32_t NF = F < f.n_features ? F : f.n_features;
     const uint64_t tiles = (n + p.R - 1) / p.R;
-    {
-        // warp items: row groups x feature chunks, about 32 warps per SM
-        const uint32_t wr = f.bins16 ? 64u : 128u;
-        const uint64_t groups = (n + wr - 1) / wr;
-        const uint64_t want = sm_count() * 32u;
-        const uint64_t fgs = (NF + BIN_F - 1) / BIN_F;
-        uint64_t n_fc = groups >= want ? 1 : (want + groups - 1) / groups;
-        if (n_fc > fgs) n_fc = fgs;
-        if (n_fc < 1) n_fc = 1;
-        const uint32_t FC = (uint32_t)((fgs + n_fc - 1) / n_fc) * BIN_F;
-        const uint64_t items = groups * ((NF + FC - 1) / FC);
-        const uint64_t blocks = (items + BIN_THREADS / 32u - 1) / (BIN_THREADS / 32u);
-        const unsigned grid = (unsigned)(blocks < sm_count() * 4u ? blocks : sm_count() * 4u);
-        const size_t smem = (predict_spl_floats(NF) + (size_t)(BIN_THREADS / 32u) * wr * BIN_XS_LD) * sizeof(float);
-        if (f.bins16)
-            launch_k(k_bin_rows<uint16_t>, grid, BIN_THREADS, smem, st, f, x, n, F, p.R, FC, static_cast<uint32_t*>(scratch));
-        else
-            launch_k(k_bin_rows<uint8_t>, grid, BIN_THREADS, smem, st, f, x, n, F, p.R, FC, static_cast<uint32_t*>(scratch));
-    }
+    if (f.bins16)
+        feature_major ? launch_bin_rows<uint16_t, true>(f, x, n, F, p.R, scratch, st)
+                      : launch_bin_rows<uint16_t, false>(f, x, n, F, p.R, scratch, st);
+    else
+        feature_major ? launch_bin_rows<uint8_t, true>(f, x, n, F, p.R, scratch, st)
+                      : launch_bin_rows<uint8_t, false>(f, x, n, F, p.R, scratch, st);
     const unsigned grid = (unsigned)(tiles < sm_count() ? tiles : sm_count());
     const unsigned threads = p.R * p.S;
     const unsigned char* bg = static_cast<const unsigned char*>(scratch);
@@ -4829,8 +4887,6 @@ void init_kernel_attributes() {
     if (cudaGetDevice(&dev) != cudaSuccess) return;
     const unsigned long long bit = dev < 64 ? (1ull << dev) : 0ull;
     if (bit && (done.load() & bit)) return;
-    cudaFuncSetAttribute(k_bin_rows<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-    cudaFuncSetAttribute(k_bin_rows<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     cudaFuncSetAttribute(k_predict_heap<true, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
     cudaFuncSetAttribute(k_predict_heap<false, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
     cudaFuncSetAttribute(k_predict_heap<false, uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);

@@ -608,10 +608,11 @@ uint32_t predict_heap_rows(const HeapForest& f, uint32_t n_features, uint64_t n)
 size_t predict_heap_scratch(const HeapForest& f, uint32_t n_features, uint64_t n);
 size_t predict_heap_scratch_max(const HeapForest& f, uint32_t n_features, uint64_t n_max);
 constexpr uint32_t PREDICT_TILE_MAX = 768;  // largest traversal tile (rows)
-// out [n_groups][n] raw margins of sample-major rows x [n][n_features];
-// scratch: predict_heap_scratch bytes of device memory (16-byte aligned).
-void launch_predict_heap(const HeapForest& f, const float* x, uint64_t n, uint32_t n_features, float* out,
-                         void* scratch, cudaStream_t st);
+// out [n_groups][n] raw margins of sample-major rows x [n][n_features]
+// (feature_major != 0: x [n_features][n]); scratch: predict_heap_scratch
+// bytes of device memory (16-byte aligned).
+void launch_predict_heap(const HeapForest& f, const float* x, uint64_t n, uint32_t n_features, int feature_major,
+                         float* out, void* scratch, cudaStream_t st);
 // transform: 1 sigmoid, 2 softmax over [G][n]
 void launch_transform(int transform, float* out, uint32_t G, uint64_t n, cudaStream_t st);
 // a[i] = a[i] + b[i] (f32), i < n
