@@ -124,11 +124,11 @@ struct DeviceForest {
     DevArray<uint8_t> heap_finfo;
     HeapForest heap{};
 };
-// out [n_groups][n] raw margins of sample-major rows x [n][F] (device). The
-// shared-memory traversal bins the rows into scratch first: the caller's
+// out [n_groups][n] raw margins of sample-major rows x [n][F] (device;
+// feature_major: x [F][n]). The shared-memory traversal bins the rows into scratch first: the caller's
 // (scratch_bytes >= what n rows need) or stream-ordered pool memory.
 void forest_predict_rows(const DeviceForest& f, const float* x, uint64_t n, uint64_t F, float* out, cudaStream_t st,
-                         void* scratch = nullptr, size_t scratch_bytes = 0);
+                         void* scratch = nullptr, size_t scratch_bytes = 0, bool feature_major = false);
 bool forest_uses_heap(const DeviceForest& f, uint64_t n, uint64_t F);
 // Node-list forest of `trees` (forest order; no heap copy) into f.
 void upload_node_forest(const std::vector<const HostTree*>& trees, uint32_t n_groups, const std::vector<float>& base,
