@@ -1247,12 +1247,15 @@ k_b_hist_part_tma(BDev d, const LaneTile* __restrict__ tiles, uint32_t n_tiles, 
                   GradRef gr, uint32_t n_rows, void* __restrict__ part, const __grid_constant__ CUtensorMap m32,
                   const __grid_constant__ CUtensorMap m16) {
     BST_PDL_ENTER();
-    extern __shared__ __align__(128) unsigned char smem_raw[];
+    // a name of its own: extern shared arrays of one name share one symbol,
+    // whose alignment is that of whichever declaration the compiler meets
+    // last, and the copies' destinations need 128 bytes
+    extern __shared__ __align__(128) unsigned char tma_smem[];
     constexpr uint32_t NW = acc_words(MODE);
     constexpr uint32_t plane = LANE_ROWS * 32u;
-    uint32_t* sm = reinterpret_cast<uint32_t*>(smem_raw);
+    uint32_t* sm = reinterpret_cast<uint32_t*>(tma_smem);
     const uint32_t nwarps = blockDim.x >> 5;
-    uint8_t* stage = smem_raw + NW * plane * 4u;  // 128-byte aligned (plane bytes are)
+    uint8_t* stage = tma_smem + NW * plane * 4u;  // 128-byte aligned (plane bytes are)
     uint64_t* bars = reinterpret_cast<uint64_t*>(stage + (size_t)nwarps * LANE_TMA_STAGES * LANE_TMA_STAGE);
     __shared__ LaneTile tile;
     using E = typename PartEntry<MODE>::T;
