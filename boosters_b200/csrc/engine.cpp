@@ -3263,14 +3263,14 @@ void forest_predict_rows(const DeviceForest& f, const float* x, uint64_t n, uint
         launch_predict(f.view, x, n, (uint32_t)F, feature_major ? 1 : 0, out, st);
         return;
     }
-    const size_t need = predict_heap_scratch(f.heap, (uint32_t)F, n);
-    if (scratch && scratch_bytes >= need) {
-        launch_predict_heap(f.heap, x, n, (uint32_t)F, feature_major ? 1 : 0, out, scratch, st);
+    if (scratch && scratch_bytes >= predict_heap_scratch_min(f.heap, (uint32_t)F, n)) {
+        launch_predict_heap(f.heap, x, n, (uint32_t)F, feature_major ? 1 : 0, out, scratch, scratch_bytes, st);
         return;
     }
+    const size_t need = std::max<size_t>(predict_heap_scratch(f.heap, (uint32_t)F, n), 16);
     void* tmp = nullptr;
-    BST_CK(cudaMallocFromPoolAsync(&tmp, std::max<size_t>(need, 16), scratch_pool(), st));
-    launch_predict_heap(f.heap, x, n, (uint32_t)F, feature_major ? 1 : 0, out, tmp, st);
+    BST_CK(cudaMallocFromPoolAsync(&tmp, need, scratch_pool(), st));
+    launch_predict_heap(f.heap, x, n, (uint32_t)F, feature_major ? 1 : 0, out, tmp, need, st);
     BST_CK(cudaFreeAsync(tmp, st));
 }
 

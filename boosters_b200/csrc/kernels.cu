@@ -4459,13 +4459,58 @@ static HeapPlan heap_plan(const HeapForest& f, uint32_t F, uint64_t n) {
 
 uint32_t predict_heap_rows(const HeapForest& f, uint32_t F, uint64_t n) { return heap_plan(f, F, n).R; }
 
+// Small batches: the trees split over blocks. Without it one block per
+// 128-row tile walks the whole forest (1000 trees of depth 8: 88 us for any
+// batch of up to 148 tiles). The blocks of a tile each take SPLIT_TREES
+// trees or fewer, leave every tree's leaf values in global memory, and
+// k_heap_sum adds them in forest order (the same f32 additions). Worth it
+// from SPLIT_MIN_TREES trees on (below, the walk is shorter than the extra
+// launch) while each tile is the smallest (every SM has one tile or less)
+// and the values, 4 bytes per row and tree, stay within SPLIT_MAX_VALUES.
+// Whole calls on device rows of 100 features, before -> now: 16 rows x 1000
+// trees 94 -> 24 us, 4,096 x 1000 98 -> 35, 10,000 x 1000 114 -> 65, 8,000 x
+// 96 32 -> 25; 18,900 x 1000 (past the limit) 118 -> 121.
+constexpr uint32_t SPLIT_TREES = 16;
+constexpr uint32_t SPLIT_MIN_TREES = 96;
+constexpr uint64_t SPLIT_MAX_VALUES = 12ull << 20;
+constexpr uint32_t SPLIT_THREADS = 256;
+constexpr uint32_t SUM_CHUNK = 256;  // trees staged per step of k_heap_sum
+
+struct SplitPlan {
+    uint32_t trees = 0;  // per block; 0: not split
+    size_t smem = 0, values = 0;  // values: floats of leaf values
+};
+
+static SplitPlan split_plan(const HeapForest& f, const HeapPlan& p, uint64_t n) {
+    SplitPlan s;
+    if (p.R != PREDICT_MIN_ROWS || f.n_trees < SPLIT_MIN_TREES) return s;
+    const uint64_t tiles = (n + p.R - 1) / p.R;
+    const uint64_t rows = tiles * p.R;
+    if (tiles > sm_count() || rows * f.n_trees > SPLIT_MAX_VALUES) return s;
+    // about four blocks per SM; at least four trees (the chains of a warp)
+    uint64_t t = (f.n_trees * tiles + sm_count() * 4u - 1) / (sm_count() * 4u);
+    t = (t + PREDICT_IL - 1) / PREDICT_IL * PREDICT_IL;
+    s.trees = (uint32_t)(t < PREDICT_IL ? PREDICT_IL : (t > SPLIT_TREES ? SPLIT_TREES : t));
+    s.smem = (size_t)s.trees * PREDICT_TREE_BYTES + p.col_bytes;  // <= PREDICT_SMEM, as the plan's
+    s.values = (size_t)rows * f.n_trees;
+    return s;
+}
+
+static size_t tile_bytes(const HeapPlan& p, uint64_t n) {
+    return p.R ? ((size_t)((n + p.R - 1) / p.R) * p.col_bytes + 255u) & ~(size_t)255u : 0;
+}
+
+size_t predict_heap_scratch_min(const HeapForest& f, uint32_t F, uint64_t n) {
+    return tile_bytes(heap_plan(f, F, n), n);
+}
+
 size_t predict_heap_scratch(const HeapForest& f, uint32_t F, uint64_t n) {
     const HeapPlan p = heap_plan(f, F, n);
-    return p.R ? (size_t)((n + p.R - 1) / p.R) * p.col_bytes : 0;
+    return tile_bytes(p, n) + split_plan(f, p, n).values * sizeof(float);
 }
 
 size_t predict_heap_scratch_max(const HeapForest& f, uint32_t F, uint64_t n_max) {
-    return (size_t)(n_max + PREDICT_MAX_ROWS) * f.n_cols * (f.bins16 ? 2u : 1u);
+    return (size_t)(n_max + PREDICT_MAX_ROWS) * f.n_cols * (f.bins16 ? 2u : 1u) + 256u;
 }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -4778,27 +4823,123 @@ k_predict_heap(HeapForest f, const unsigned char* __restrict__ bins_g, uint64_t 
     }
 }
 
+// Leaf values of one slice of trees for one tile: lv[tree][row] (ld rows per
+// tree), trees in the forest's group order. Warps take (row group, four
+// trees) pairs. Bound by latency: one load of the tile and the trees, then
+// 8 dependent pairs of shared-memory reads.
+template <bool CAT, typename BinT>
+__global__ void __launch_bounds__(SPLIT_THREADS)
+k_heap_leaves(HeapForest f, const unsigned char* __restrict__ bins_g, uint64_t n, uint32_t R, uint32_t slice,
+              uint32_t ld, float* __restrict__ lv) {
+    BST_PDL_ENTER();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t* tb = reinterpret_cast<const uint32_t*>(smem_raw);  // [slice][HEAP_NODES]
+    unsigned char* bins = smem_raw + (size_t)slice * PREDICT_TREE_BYTES;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t tile = blockIdx.x, t0 = blockIdx.y * slice;
+    const uint32_t nt = min(slice, f.n_trees - t0);
+    const uint32_t Rb = R * (uint32_t)sizeof(BinT);
+    const uint32_t col_bytes = f.n_cols * Rb;
+    const uint32_t r0 = tile * R;
+    const uint32_t nr = (uint32_t)min((uint64_t)R, n - r0);
+    {
+        const uint4* src = reinterpret_cast<const uint4*>(f.nodes + (size_t)t0 * HEAP_NODES);
+        uint4* dst = reinterpret_cast<uint4*>(smem_raw);
+        for (uint32_t i = tid; i < nt * (PREDICT_TREE_BYTES / 16u); i += SPLIT_THREADS) cp_async16(dst + i, src + i);
+        const uint4* bsrc = reinterpret_cast<const uint4*>(bins_g + (size_t)tile * col_bytes);
+        uint4* bdst = reinterpret_cast<uint4*>(bins);
+        for (uint32_t i = tid; i < col_bytes / 16u; i += SPLIT_THREADS) cp_async16(bdst + i, bsrc + i);
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const uint32_t nrg = (nr + 31u) / 32u, quads = (nt + PREDICT_IL - 1) / PREDICT_IL;
+    for (uint32_t p = warp; p < nrg * quads; p += SPLIT_THREADS / 32u) {
+        const uint32_t rg = (p % nrg) * 32u + lane, q0 = p / nrg * PREDICT_IL;
+        const unsigned char* cb = bins + (sizeof(BinT) == 1 ? (rg >> 7) * 128u + 4u * lane + ((rg >> 5) & 3u)
+                                                            : (rg >> 6) * 128u + 4u * lane + 2u * ((rg >> 5) & 1u));
+        float* o = lv + (size_t)t0 * ld + r0 + rg;
+        heap_walk<CAT, BinT>(tb, q0, min(q0 + PREDICT_IL, nt), cb, Rb, f,
+                             [&](uint32_t q, float v) { o[(size_t)q * ld] = v; });
+    }
+}
+
+// out[g][row] = base[g] + the trees' leaf values in forest order: a block
+// stages SUM_CHUNK trees of 32 rows at a time (two buffers), one warp adds.
+// The f32 chain of additions bounds it (1000 trees: 2 us of 4-cycle adds).
+__global__ void __launch_bounds__(SPLIT_THREADS)
+k_heap_sum(HeapForest f, const float* __restrict__ lv, uint32_t ld, uint64_t n, float* __restrict__ out) {
+    BST_PDL_ENTER();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float* buf = reinterpret_cast<float*>(smem_raw);  // [2][SUM_CHUNK][32]
+    const uint32_t tid = threadIdx.x, g = blockIdx.y, r0 = blockIdx.x * 32u;
+    const uint32_t t0 = f.group_off[g], t1 = f.group_off[g + 1];
+    const uint32_t n_chunks = (t1 - t0 + SUM_CHUNK - 1) / SUM_CHUNK;
+    auto issue = [&](uint32_t c) {
+        const uint32_t ta = t0 + c * SUM_CHUNK, nt = min(SUM_CHUNK, t1 - ta);
+        float* dst = buf + (size_t)(c & 1u) * SUM_CHUNK * 32u;
+        for (uint32_t i = tid; i < nt * 8u; i += SPLIT_THREADS)
+            cp_async16(dst + i * 4u, lv + (size_t)(ta + i / 8u) * ld + r0 + (i & 7u) * 4u);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc = f.base[g];
+    if (n_chunks) issue(0);
+    for (uint32_t c = 0; c < n_chunks; ++c) {
+        if (c + 1 < n_chunks) {
+            issue(c + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        if (tid < 32u) {
+            const float* v = buf + (size_t)(c & 1u) * SUM_CHUNK * 32u + tid;
+            const uint32_t nt = min(SUM_CHUNK, t1 - t0 - c * SUM_CHUNK);
+#pragma unroll 16
+            for (uint32_t q = 0; q < nt; ++q) acc = acc + v[q * 32u];
+        }
+        __syncthreads();  // the buffer is free for chunk c + 2
+    }
+    if (tid < 32u && (uint64_t)r0 + tid < n) out[(uint64_t)g * n + r0 + tid] = acc;
+}
+
+template <bool CAT, typename BinT>
+static void launch_heap(const HeapForest& f, const HeapPlan& p, const SplitPlan& sp, const unsigned char* bins,
+                        float* lv, uint64_t n, float* out, cudaStream_t st) {
+    const uint64_t tiles = (n + p.R - 1) / p.R;
+    if (sp.trees) {
+        const uint32_t ld = (uint32_t)tiles * p.R;
+        launch_k(k_heap_leaves<CAT, BinT>, dim3((unsigned)tiles, (f.n_trees + sp.trees - 1) / sp.trees), SPLIT_THREADS,
+                 sp.smem, st, f, bins, n, p.R, sp.trees, ld, lv);
+        launch_k(k_heap_sum, dim3((unsigned)((n + 31) / 32), f.n_groups), SPLIT_THREADS, 2u * SUM_CHUNK * 32u * 4u, st, f,
+                 static_cast<const float*>(lv), ld, n, out);
+        return;
+    }
+    const unsigned grid = (unsigned)(tiles < sm_count() ? tiles : sm_count());
+    launch_k(k_predict_heap<CAT, BinT>, grid, p.R * p.S, p.smem, st, f, bins, n, p.R, p.S, out);
+}
+
 void launch_predict_heap(const HeapForest& f, const float* x, uint64_t n, uint32_t F, int feature_major, float* out,
-                         void* scratch, cudaStream_t st) {
+                         void* scratch, size_t scratch_bytes, cudaStream_t st) {
     if (n == 0) return;
     init_kernel_attributes();  // per device: the kernels' shared-memory opt-in
     const HeapPlan p = heap_plan(f, F, n);
-    const uint64_t tiles = (n + p.R - 1) / p.R;
     if (f.bins16)
         feature_major ? launch_bin_rows<uint16_t, true>(f, x, n, F, p.R, scratch, st)
                       : launch_bin_rows<uint16_t, false>(f, x, n, F, p.R, scratch, st);
     else
         feature_major ? launch_bin_rows<uint8_t, true>(f, x, n, F, p.R, scratch, st)
                       : launch_bin_rows<uint8_t, false>(f, x, n, F, p.R, scratch, st);
-    const unsigned grid = (unsigned)(tiles < sm_count() ? tiles : sm_count());
-    const unsigned threads = p.R * p.S;
     const unsigned char* bg = static_cast<const unsigned char*>(scratch);
+    const size_t tb = tile_bytes(p, n);
+    SplitPlan sp = split_plan(f, p, n);
+    if (tb + sp.values * sizeof(float) > scratch_bytes) sp = SplitPlan{};  // no room for the values
+    float* lv = reinterpret_cast<float*>(static_cast<unsigned char*>(scratch) + tb);
     if (f.has_cat)
-        launch_k(k_predict_heap<true, uint16_t>, grid, threads, p.smem, st, f, bg, n, p.R, p.S, out);
+        launch_heap<true, uint16_t>(f, p, sp, bg, lv, n, out, st);
     else if (f.bins16)
-        launch_k(k_predict_heap<false, uint16_t>, grid, threads, p.smem, st, f, bg, n, p.R, p.S, out);
+        launch_heap<false, uint16_t>(f, p, sp, bg, lv, n, out, st);
     else
-        launch_k(k_predict_heap<false, uint8_t>, grid, threads, p.smem, st, f, bg, n, p.R, p.S, out);
+        launch_heap<false, uint8_t>(f, p, sp, bg, lv, n, out, st);
 }
 
 __global__ void k_transform(int t, float* __restrict__ p, uint32_t G, uint64_t n) {
@@ -4895,6 +5036,10 @@ void init_kernel_attributes() {
     cudaFuncSetAttribute(k_predict_heap<true, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
     cudaFuncSetAttribute(k_predict_heap<false, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
     cudaFuncSetAttribute(k_predict_heap<false, uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
+    cudaFuncSetAttribute(k_heap_leaves<true, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
+    cudaFuncSetAttribute(k_heap_leaves<false, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
+    cudaFuncSetAttribute(k_heap_leaves<false, uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREDICT_SMEM);
+    cudaFuncSetAttribute(k_heap_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2u * SUM_CHUNK * 32u * 4u));
     const int hist_smem = 200 * 1024;
     cudaFuncSetAttribute(k_hist_build<GRAD_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, hist_smem);
     cudaFuncSetAttribute(k_hist_build<GRAD_Q16>, cudaFuncAttributeMaxDynamicSharedMemorySize, hist_smem);

@@ -603,16 +603,18 @@ struct HeapForest {
 // Rows per block of the shared-memory traversal for n rows of F features (0:
 // the forest does not fit; use the node-list traversal).
 uint32_t predict_heap_rows(const HeapForest& f, uint32_t n_features, uint64_t n);
-// Bytes of bin-tile scratch the traversal of n rows needs; an upper bound for
-// any n <= n_max.
+// Bytes of scratch the traversal of n rows uses (bin tiles, and for small
+// batches the trees' leaf values); the least it can run with (bin tiles); an
+// upper bound of the least for any n <= n_max.
 size_t predict_heap_scratch(const HeapForest& f, uint32_t n_features, uint64_t n);
+size_t predict_heap_scratch_min(const HeapForest& f, uint32_t n_features, uint64_t n);
 size_t predict_heap_scratch_max(const HeapForest& f, uint32_t n_features, uint64_t n_max);
 constexpr uint32_t PREDICT_TILE_MAX = 768;  // largest traversal tile (rows)
 // out [n_groups][n] raw margins of sample-major rows x [n][n_features]
-// (feature_major != 0: x [n_features][n]); scratch: predict_heap_scratch
-// bytes of device memory (16-byte aligned).
+// (feature_major != 0: x [n_features][n]); scratch: predict_heap_scratch_min
+// bytes of device memory or more (256-byte aligned).
 void launch_predict_heap(const HeapForest& f, const float* x, uint64_t n, uint32_t n_features, int feature_major,
-                         float* out, void* scratch, cudaStream_t st);
+                         float* out, void* scratch, size_t scratch_bytes, cudaStream_t st);
 // transform: 1 sigmoid, 2 softmax over [G][n]
 void launch_transform(int transform, float* out, uint32_t G, uint64_t n, cudaStream_t st);
 // a[i] = a[i] + b[i] (f32), i < n
