@@ -798,6 +798,8 @@ class Trainer {
             if (qmode_ != GRAD_F32) {  // the quantisation also writes the fixed-point scales
                 launch_quantize(qmode_, G_, gh_.p, n_, maxabs_.p, cfg_.seed, round_no_, 0u, gq_.p, qscales_.p, st_,
                                 scales_.p);
+            } else if (use_small_) {
+                launch_fixed_values(maxabs_.p, G_, n_, gh_.p, scales_.p, small_fix_.p, st_);
             } else {
                 launch_fixed_scales(maxabs_.p, G_, n_, scales_.p, st_);
             }
@@ -1205,7 +1207,8 @@ class Trainer {
         d_sums_.alloc(2 * ((size_t)max_pnodes_ + 1));
         d_leaves_.alloc(max_pnodes_ + 1);
         stage_.reserve(max_chunks * 48 + (size_t)(max_pnodes_ + 4) * 256 + (1 << 20));
-        if (n_cols_) setup_hist_state();
+        use_small_ = small_tree_applies();
+        if (n_cols_ && !use_small_) setup_hist_state();
         n_sampled_.assign(G_, (uint32_t)n_);
         goss_ = !external_ && cfg_.goss_top_rate > 0.0f;
         goss_warmup_ = (uint64_t)(1.0f / cfg_.learning_rate);  // row.rs:112-116
@@ -1226,9 +1229,13 @@ class Trainer {
         use_batched_ = cfg_.batched && !leafwise_ && n_cols_ > 0 && cfg_.max_depth <= 14;
         spec_leafwise_ = cfg_.batched && leafwise_ && n_cols_ > 0;
         if (use_batched_ || spec_leafwise_) {
-            if (use_batched_) setup_batched();
+            if (use_small_)
+                setup_small();
+            else if (use_batched_)
+                setup_batched();
             if (spec_leafwise_) setup_lw_device();
-            for (auto& q : qpos_) q.alloc((size_t)n_ * grad_bytes());
+            if (!use_small_)
+                for (auto& q : qpos_) q.alloc((size_t)n_ * grad_bytes());
             if (p_.f8) fm8_.alloc((size_t)n_ * p_.f8);
             if (p_.f16) fm16_.alloc((size_t)n_ * p_.f16);
             launch_transpose_bins(b_.bins8, p_.s8, p_.f8, b_.bins16, p_.s16, p_.f16, n_, fm8_.p, fm16_.p, st_);
@@ -1236,6 +1243,149 @@ class Trainer {
             fm_ = BinsFM{fm8_.p, fm16_.p, n_};
         }
         setup_renew();
+    }
+
+    // ---- small training sets: one cooperative launch per tree (small_tree.cuh) --
+    // us per tree, one launch / level kernels (logistic, depth 6 unless said):
+    // 5,000 x 100 fp32 124 / 263, q8 122 / 248; 50,000 x 100 fp32 249 / 299,
+    // q8 206 / 275, depth 8 430 / 465; 20,000 x 300 (three columns a block)
+    // 371 / 373; 100,000 x 100 fp32 378 / 318, q8 295 / 296. The row loop of
+    // the one launch grows with the rows, so the line is drawn where fp32
+    // crosses.
+    static constexpr uint64_t SMALL_TREE_ROWS = 70000;
+    bool use_small_ = false;
+    DevArray<uint8_t> small_buf_;  // zeroed scratch, then BState and the tree
+    DevArray<uint16_t> small_rt_;
+    DevArray<long long> small_tot_;
+    DevArray<longlong2> small_fix_;  // f32 form: the round's gradients in fixed point
+    size_t small_zero_ = 0, small_out_ = 0, small_out_bytes_ = 0;
+    SmallTree small_{};
+
+    // Depth-wise batched trees of up to SMALL_TREE_DEPTH levels, without leaf
+    // renewing (it needs the rows grouped by leaf), per-phase timers (they
+    // time the level kernels) or a launch-shape cache file (it names the level
+    // kernels' shapes), while the rows a level reads are few enough.
+    bool small_tree_applies() const {
+        if (!(cfg_.batched && !leafwise_ && n_cols_ > 0) || external_ || cfg_.max_depth == 0 ||
+            cfg_.max_depth > SMALL_TREE_DEPTH || cfg_.phase_timings || cfg_.autotune_cache ||
+            cfg_.objective == BST_OBJ_ABSOLUTE || cfg_.objective == BST_OBJ_PINBALL)
+            return false;
+        // a block reads every row once per level and column of its own
+        const uint64_t per_block = (n_cols_ + sm_count() - 1) / sm_count();
+        if (n_ * per_block > SMALL_TREE_ROWS) return false;
+        uint32_t max_bins = 1;
+        bool cat = false;
+        for (uint32_t c = 0; c < n_cols_; ++c) {
+            max_bins = std::max(max_bins, p_.col_nbins[c]);
+            cat = cat || p_.col_cat[c];
+        }
+        return small_tree_fits(qmode_, n_, max_bins, cat);
+    }
+
+    void setup_small() {
+        const uint32_t nodes = 1u << cfg_.max_depth;  // leaves, and entries of the per-node arrays
+        max_tnodes_ = 2 * nodes;
+        m_.tune_info = "one launch per tree (built-in)";
+        size_t off = 0;
+        auto take = [&](size_t bytes) {
+            const size_t at = off;
+            off += (bytes + 63) & ~size_t(63);
+            return at;
+        };
+        const size_t o_bar = take(64), o_keys = take(8 * (size_t)nodes), o_cnt = take(4 * (size_t)nodes),
+                     o_scnt = take(4 * (size_t)nodes), o_x = take(16 * (size_t)max_tnodes_);
+        small_out_ = take(sizeof(BState));
+        small_zero_ = off;
+        const size_t o_tree = take(sizeof(BTreeNode) * max_tnodes_);
+        small_out_bytes_ = off - small_out_;
+        small_buf_.alloc(off);
+        small_rt_.alloc(n_);
+        small_tot_.alloc(2 * (size_t)nodes);
+        if (qmode_ == GRAD_F32) small_fix_.alloc((size_t)G_ * n_);
+        std::vector<BColumn> bc(n_cols_);
+        bool cat = false;
+        for (uint32_t c = 0; c < n_cols_; ++c) {
+            bc[c] = BColumn{p_.col_matrix[c], p_.col_pos[c], p_.col_missing[c], p_.col_default[c]};
+            cat = cat || p_.col_cat[c];
+        }
+        d_bcols_.alloc(n_cols_);
+        BST_CK(cudaMemcpy(d_bcols_.p, bc.data(), sizeof(BColumn) * n_cols_, cudaMemcpyHostToDevice));
+        for (auto& sl : slots_) {
+            sl.small = static_cast<char*>(pinned_alloc(small_out_bytes_));
+            BST_CK(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
+        }
+        uint8_t* b = small_buf_.p;
+        SmallTree& a = small_;
+        a.n = (uint32_t)n_;
+        a.n_cols = n_cols_;
+        a.max_depth = cfg_.max_depth;
+        a.cols = scan_cols_.p;
+        a.bcols = d_bcols_.p;
+        a.has_cat = cat ? 1 : 0;
+        a.last_wins = last_wins_ ? 1 : 0;
+        a.gp = gp_;
+        a.lp = LeafParams{(double)cfg_.lambda, (double)cfg_.alpha, (double)cfg_.min_gain, cfg_.learning_rate, 0u};
+        a.hist = hist_.p;
+        a.slot_bins = slot_bins_;
+        a.cand = d_cand_.p;
+        a.rt = small_rt_.p;
+        a.tot = small_tot_.p;
+        a.bar = reinterpret_cast<uint32_t*>(b + o_bar);
+        a.keys = reinterpret_cast<unsigned long long*>(b + o_keys);
+        a.cnt = reinterpret_cast<uint32_t*>(b + o_cnt);
+        a.scnt = reinterpret_cast<uint32_t*>(b + o_scnt);
+        a.xsum = reinterpret_cast<unsigned long long*>(b + o_x);
+        a.state = reinterpret_cast<BState*>(b + small_out_);
+        a.tree = reinterpret_cast<BTreeNode*>(b + o_tree);
+        a.row_leaf = cfg_.record_leaves ? row_leaf_.p : nullptr;
+    }
+
+    // Enqueues the tree of output o into ring slot `si` (no host wait).
+    void launch_small(uint32_t o, uint32_t si) {
+        BST_RANGE("bst.tree");
+        Slot& sl = slots_[si];
+        upload_col_masks(o, si);
+        SmallTree a = small_;
+        a.n_root = n_sampled_[o];
+        a.fm8 = fm8_.p;
+        a.fm16 = fm16_.p;
+        a.gr = grad_ref(o);
+        a.fix = small_fix_.p + (qmode_ == GRAD_F32 ? (size_t)o * n_ : 0);
+        a.fscale = scales_.p + 4 * (size_t)o;
+        a.scale = unit_scale(o);
+        a.colmask = colmask();
+        a.rmask = rowmask(o);
+        a.pred = pred_.p + (size_t)o * n_;
+        BST_CK(cudaMemsetAsync(small_buf_.p, 0, small_zero_, st_));
+        launch_small_tree(a, st_);
+        BST_CK(cudaMemcpyAsync(sl.small, small_buf_.p + small_out_, small_out_bytes_, cudaMemcpyDeviceToHost, st_));
+        if (cfg_.record_leaves) {
+            sl.row_leaf.resize(n_);
+            BST_CK(cudaMemcpyAsync(sl.row_leaf.data(), row_leaf_.p, sizeof(uint32_t) * n_, cudaMemcpyDeviceToHost, st_));
+        }
+        BST_CK(cudaEventRecord(sl.done, st_));
+        sl.pending = true;
+        sl.o = o;
+    }
+
+    HostTree collect_small(uint32_t si) {
+        Slot& sl = slots_[si];
+        BST_CK(cudaEventSynchronize(sl.done));
+        BST_CK(cudaGetLastError());
+        sl.pending = false;
+        HostTree t;
+        t.group = sl.o;
+        t.row_leaf = std::move(sl.row_leaf);
+        sl.row_leaf = {};
+        const BState* st = reinterpret_cast<const BState*>(sl.small);
+        if (st->err || st->n_tnodes == 0 || st->n_tnodes > max_tnodes_)
+            throw Error{BST_ERR_CUDA, "a tree kernel's bounded wait for its blocks gave up; the tree is invalid"};
+        m_.counters.launches += 1;
+        m_.counters.hist_launches += 1;
+        m_.counters.hist_rows += st->hist_rows;
+        m_.counters.hist_bytes += st->hist_rows * ((uint64_t)p_.f8 + 2ull * p_.f16 + grad_bytes() + 4ull);
+        m_.counters.scan_launches += 1;
+        return host_tree_from(std::move(t), st->n_tnodes, reinterpret_cast<const BTreeNode*>(sl.small + sizeof(BState)));
     }
 
     // ---- device-side level loop, one CUDA graph per output (kernels.h) -------
@@ -1269,6 +1419,7 @@ class Trainer {
     struct Slot {
         BTreeNode* tree = nullptr;  // pinned
         BState* state = nullptr;    // pinned
+        char* small = nullptr;      // pinned: BState, then the tree (launch_small)
         cudaEvent_t done = nullptr, w0 = nullptr, w1 = nullptr;
         bool pending = false;
         uint32_t o = 0;
@@ -1290,6 +1441,7 @@ class Trainer {
         for (auto& sl : slots_) {
             pinned_free(sl.tree);
             pinned_free(sl.state);
+            pinned_free(sl.small);
             for (auto e : {sl.done, sl.w0, sl.w1})
                 if (e) cudaEventDestroy(e);
         }
@@ -1631,6 +1783,7 @@ class Trainer {
 
     // Enqueues the tree of output o into ring slot `si` (no host wait).
     void launch_batched(uint32_t o, uint32_t si) {
+        if (use_small_) return launch_small(o, si);
         BST_RANGE("bst.tree");  // the tree's graph launch (its kernels run after the range closes)
         Slot& sl = slots_[si];
         const size_t gi = (size_t)o * RING + si;
@@ -1688,6 +1841,7 @@ class Trainer {
 
     // Waits for ring slot `si` and converts its device tree to a host tree.
     HostTree collect_batched(uint32_t si) {
+        if (use_small_) return collect_small(si);
         Slot& sl = slots_[si];
         const uint32_t o = sl.o;
         const size_t gi = (size_t)o * RING + si;

@@ -425,10 +425,8 @@ void launch_gradients(int objective, uint32_t G, const float* pred, const float*
                                                                           alpha, delta);
 }
 
-// Fixed-point scale of element i (output i / 2, grad or hess i % 2).
-__device__ void write_fixed_scale(const unsigned* __restrict__ maxabs, uint32_t i, uint64_t n,
-                                  double* __restrict__ scales) {
-    const float m = __uint_as_float(maxabs[i]);
+// Binary exponent of the fixed-point scale of values up to m in magnitude.
+__device__ int fixed_exponent(float m, uint64_t n) {
     int k = 0;
     if (m > 0.0f) {
         int e, en;
@@ -443,6 +441,13 @@ __device__ void write_fixed_scale(const unsigned* __restrict__ maxabs, uint32_t 
         if (k > 1000) k = 1000;
         if (k < -1000) k = -1000;
     }
+    return k;
+}
+
+// Fixed-point scale of element i (output i / 2, grad or hess i % 2).
+__device__ void write_fixed_scale(const unsigned* __restrict__ maxabs, uint32_t i, uint64_t n,
+                                  double* __restrict__ scales) {
+    const int k = fixed_exponent(__uint_as_float(maxabs[i]), n);
     const uint32_t o = i >> 1, which = i & 1;
     scales[4 * o + which] = ldexp(1.0, k);
     scales[4 * o + 2 + which] = ldexp(1.0, -k);
@@ -453,6 +458,36 @@ __global__ void k_fixed_scales(const unsigned* __restrict__ maxabs, uint32_t G, 
     BST_PDL_ENTER();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 2 * G) write_fixed_scale(maxabs, i, n, scales);
+}
+
+// The pairs converted once per round (the conversions from and to 64-bit
+// types run at 16 a clock and SM: converted by every column's row loop they
+// took 8 of its 22 cycles per warp and row). blockIdx.y: output.
+__global__ void __launch_bounds__(256)
+k_fixed_values(const unsigned* __restrict__ maxabs, uint32_t G, uint64_t n, const float2* __restrict__ gh,
+               double* __restrict__ scales, longlong2* __restrict__ fix) {
+    BST_PDL_ENTER();
+    __shared__ double sc[2];
+    const uint32_t o = blockIdx.y;
+    if (threadIdx.x < 2) {
+        const uint32_t i = 2 * o + threadIdx.x;
+        sc[threadIdx.x] = ldexp(1.0, fixed_exponent(__uint_as_float(maxabs[i]), n));
+        if (blockIdx.x == 0) write_fixed_scale(maxabs, i, n, scales);
+    }
+    __syncthreads();
+    const double sg = sc[0], sh = sc[1];
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const float2 v = gh[(uint64_t)o * n + i];
+        fix[(uint64_t)o * n + i] = make_longlong2(quantize(v.x, sg), quantize(v.y, sh));
+    }
+}
+
+void launch_fixed_values(const unsigned* maxabs, uint32_t G, uint64_t n, const float2* gh, double* scales,
+                         longlong2* fix, cudaStream_t st) {
+    if (n == 0 || G == 0) return;
+    uint64_t blocks = (n + 255) / 256;
+    if (blocks > (uint64_t)sm_count() * 4) blocks = (uint64_t)sm_count() * 4;
+    launch_k(k_fixed_values, dim3((unsigned)blocks, G), 256, 0, st, maxabs, G, n, gh, scales, fix);
 }
 
 void launch_fixed_scales(const unsigned* maxabs, uint32_t G, uint64_t n, double* scales,
@@ -510,6 +545,12 @@ struct GradLoad<GRAD_Q16> {
         g = v.x;
         h = v.y;
     }
+    using Raw = uint32_t;  // one register: a pair would be taken apart (and waited for) at the load
+    __device__ __forceinline__ Raw raw(uint32_t row) const { return reinterpret_cast<const uint32_t*>(q)[row]; }
+    __device__ __forceinline__ void conv(Raw v, long long& g, long long& h) const {
+        g = (int16_t)(v & 0xFFFFu);
+        h = (int16_t)(v >> 16);
+    }
     __device__ __forceinline__ void at(uint32_t pos, uint32_t row, long long& g, long long& h) const {
         const short2 v = qp ? qp[pos] : q[row];
         g = v.x;
@@ -526,6 +567,12 @@ struct GradLoad<GRAD_Q8> {
         const char2 v = q[row];
         g = v.x;
         h = v.y;
+    }
+    using Raw = uint32_t;
+    __device__ __forceinline__ Raw raw(uint32_t row) const { return reinterpret_cast<const uint16_t*>(q)[row]; }
+    __device__ __forceinline__ void conv(Raw v, long long& g, long long& h) const {
+        g = (int8_t)(v & 0xFFu);
+        h = (int8_t)((v >> 8) & 0xFFu);
     }
     __device__ __forceinline__ void at(uint32_t pos, uint32_t row, long long& g, long long& h) const {
         const char2 v = qp ? qp[pos] : q[row];
@@ -1874,21 +1921,16 @@ constexpr int SORT_N = 256;  // categorical columns with <= 256 bins
 
 }  // namespace
 
-// One warp: best split of column `col` of node `node` (the node's histogram
-// lives in slot nd.slot); writes cand[node * n_cols + col] and, for column 0,
-// the node totals, and returns the candidate's gain (-inf: none) to every
-// lane. key / cat: this warp's SORT_N-entry shared scratch. cmask (or null):
-// the node's column mask (column sampling); a masked column has no
-// candidate.
-template <typename HB>
-__device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const ScanColumn* __restrict__ cols,
-                          uint32_t n_cols, const HB* __restrict__ hist, uint64_t slot_bins,
-                          const double* __restrict__ scale, const GainParamsDev& gp, ColCand* __restrict__ cand,
-                          long long* __restrict__ node_tot, double* key, uint32_t* cat,
-                          const uint8_t* __restrict__ cmask) {
+// One warp: best split of a column of a node whose bins' sums are ld(bin);
+// writes *out and, when tot is set, the node totals, and returns the
+// candidate's gain (-inf: none) to every lane. key / cat: this warp's
+// SORT_N-entry shared scratch. masked: the column is not among the node's
+// (column sampling): no candidate.
+template <typename HB, typename Ld>
+__device__ __forceinline__ float scan_column(Ld ld, const ScanNode& nd, const ScanColumn& cm, const double* scale,
+                                             const GainParamsDev& gp, ColCand* out, long long* tot, double* key,
+                                             uint32_t* cat, bool masked) {
     const int lane = threadIdx.x & 31;
-    const ScanColumn cm = cols[col];
-    const HB* h = hist + (size_t)nd.slot * slot_bins + cm.hist_off;
     const double ig = scale[2], ih = scale[3];
     const uint32_t nb = cm.n_bins;
     const uint32_t pc = nd.count;
@@ -1897,20 +1939,19 @@ __device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const
     using TAcc = decltype(HB{}.g);  // int for HBin32: 32-bit sums
     TAcc tg_ = 0, th_ = 0;
     for (uint32_t b = lane; b < nb; b += 32) {
-        tg_ += h[b].g;
-        th_ += h[b].h;
+        tg_ += ld(b).g;
+        th_ += ld(b).h;
     }
     long long tg = warp_sum(tg_), th = warp_sum(th_);
     if (nd.flags & 1u) {
         tg = nd.pg;
         th = nd.ph;
     }
-    if (col == 0 && lane == 0) {
-        node_tot[2 * node] = tg;
-        node_tot[2 * node + 1] = th;
+    if (tot && lane == 0) {
+        tot[0] = tg;
+        tot[1] = th;
     }
-    ColCand* out = cand + (size_t)node * n_cols + col;
-    if (cmask && !cmask[col]) {  // not among the node's sampled columns
+    if (masked) {  // not among the node's sampled columns
         if (lane == 0) {
             out->gain = -INFINITY;
             out->order = 0xFFFFFFFFu;
@@ -1934,15 +1975,15 @@ __device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const
             // find.rs:286-407: forward scan (missing right), backward scan
             // (missing left) when the column has a NaN bin (the last bin).
             const bool hm = cm.has_missing != 0;
-            const long long pm_g = tg - h[nb - 1].g, pm_h = th - h[nb - 1].h;  // P[nb-2]
+            const long long pm_g = tg - ld(nb - 1).g, pm_h = th - ld(nb - 1).h;  // P[nb-2]
             using Acc = decltype(HB{}.g);  // int for HBin32: 32-bit prefix scans
             Acc carry_g = 0, carry_h = 0;
             for (uint32_t base = 0; base < nb; base += 32) {
                 const uint32_t b = base + lane;
                 Acc vg = 0, vh = 0;
                 if (b < nb) {
-                    vg = h[b].g;
-                    vh = h[b].h;
+                    vg = ld(b).g;
+                    vh = ld(b).h;
                 }
                 const Acc Pg_ = warp_incl_scan(vg, lane) + carry_g;
                 const Acc Ph_ = warp_incl_scan(vh, lane) + carry_h;
@@ -1986,8 +2027,8 @@ __device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const
     unsigned long long cats[4] = {0ull, 0ull, 0ull, 0ull};
     if (nb >= 2 && nb <= gp.max_onehot_cats) {
         for (uint32_t c = lane; c < nb; c += 32) {  // one category left (find.rs:472)
-            const double lg = (double)h[c].g * ig, lh = (double)h[c].h * ih;
-            const double rg = (double)(tg - h[c].g) * ig, rh = (double)(th - h[c].h) * ih;
+            const double lg = (double)ld(c).g * ig, lh = (double)ld(c).h * ih;
+            const double rg = (double)(tg - ld(c).g) * ig, rh = (double)(th - ld(c).h) * ih;
             const uint32_t lc = 1, rc = sat_sub(pc, 1);
             if (ctx.valid(lh, rh, lc, rc)) {
                 const float g = ctx.gain(lg, lh, rg, rh);
@@ -2005,7 +2046,7 @@ __device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const
             bool ok = false;
             double r = 0.0;
             if (c < nb) {
-                const double gg = (double)h[c].g * ig, hh = (double)h[c].h * ih;
+                const double gg = (double)ld(c).g * ig, hh = (double)ld(c).h * ih;
                 ok = hh > 1e-10;
                 r = -gg / (hh + 1e-6);
             }
@@ -2056,8 +2097,8 @@ __device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const
                 Acc vg = 0, vh = 0;
                 if (i + 1 < m) {
                     const uint32_t c = cat[i];
-                    vg = h[c].g;
-                    vh = h[c].h;
+                    vg = ld(c).g;
+                    vh = ld(c).h;
                 }
                 const Acc Pg_ = warp_incl_scan(vg, lane) + carry_g;
                 const Acc Ph_ = warp_incl_scan(vh, lane) + carry_h;
@@ -2097,6 +2138,21 @@ __device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const
         for (int q = 0; q < 4; ++q) out->cats[q] = cats[q];
     }
     return best.gain;
+}
+
+// The same for column `col` of node `node`, whose histogram lives in slot
+// nd.slot: cand[node * n_cols + col] and, for column 0, the node totals.
+// cmask (or null): the node's column mask.
+template <typename HB>
+__device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const ScanColumn* __restrict__ cols,
+                          uint32_t n_cols, const HB* __restrict__ hist, uint64_t slot_bins,
+                          const double* __restrict__ scale, const GainParamsDev& gp, ColCand* __restrict__ cand,
+                          long long* __restrict__ node_tot, double* key, uint32_t* cat,
+                          const uint8_t* __restrict__ cmask) {
+    const ScanColumn cm = cols[col];
+    const HB* h = hist + (size_t)nd.slot * slot_bins + cm.hist_off;
+    return scan_column<HB>([h](uint32_t b) { return h[b]; }, nd, cm, scale, gp, cand + (size_t)node * n_cols + col,
+                           col == 0 ? node_tot + 2 * node : nullptr, key, cat, cmask && !cmask[col]);
 }
 
 template <typename HB>
@@ -4342,6 +4398,8 @@ void launch_leaf_renew(const BDev& d, const RenewDev& r, const uint32_t* r0, con
     launch_k(k_renew_apply, grid, 256, 0, st, d, r, lr);
 }
 
+#include "small_tree.cuh"
+
 // ============================================================================
 // K9: forest traversal (tree_view.rs:119-160, predictor.rs:271-302)
 // One thread per row; trees summed in forest order per group in f32.
@@ -5053,6 +5111,9 @@ void init_kernel_attributes() {
         for (int v = 0; v < LANE_VARIANTS; ++v)
             cudaFuncSetAttribute(lane_kernel_of(m, v), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)lane_smem_bytes(m, v));
+    for (int m = 0; m < 3; ++m)
+        for (int w = 0; w < 2; ++w)
+            cudaFuncSetAttribute(small_tree_kernel(m, w != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ST_DYN);
     cudaFuncSetAttribute(k_lw_replay<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LW_REPLAY_SMEM_MAX);
     done.fetch_or(bit);
 }

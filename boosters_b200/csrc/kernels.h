@@ -105,6 +105,9 @@ constexpr int HIST_CHUNK_MAX = 4096; // rows per block: 4096 * 2^20 < 2^32, 4096
 // scales [G][4] = (2^kg, 2^kh, 2^-kg, 2^-kh).
 void launch_fixed_scales(const unsigned* maxabs, uint32_t G, uint64_t n, double* scales,
                          cudaStream_t st);
+// The same scales, and every pair of gh [G][n] in fixed point.
+void launch_fixed_values(const unsigned* maxabs, uint32_t G, uint64_t n, const float2* gh, double* scales,
+                         longlong2* fix, cudaStream_t st);
 
 // Gradient source of the histogram and node-sum kernels (values = BST_PRECISION_*):
 //   GRAD_F32  gh (f32 pairs) as fixed point round(v * scale[0..1]), exact int64 sums
@@ -530,6 +533,43 @@ void launch_b_leaf_sums(const BDev& d, const uint32_t* r0, const uint32_t* r1, c
                         const double* scale, uint32_t grid, cudaStream_t st);
 void launch_b_leaf_update(const BDev& d, const uint32_t* r0, const uint32_t* r1, float* pred, uint32_t* row_leaf,
                           uint32_t grid, cudaStream_t st);
+
+// ---- a whole depth-wise tree in one cooperative launch (small_tree.cuh) -------
+constexpr uint32_t SMALL_TREE_DEPTH = 8;  // deepest tree
+struct SmallTree {
+    uint32_t n, n_cols, max_depth, n_root;  // n_root: rows (sampled rows) of the root
+    const uint8_t* fm8;    // column-major bins [column][n]
+    const uint16_t* fm16;
+    GradRef gr;            // row-order gradients of the histograms (its gh: the f32 pairs)
+    const longlong2* fix;  // GRAD_F32: the pairs in fixed point (launch_fixed_values)
+    const double* fscale;  // fixed-point scales of the f32 pairs (leaf sums)
+    const double* scale;   // units of the histogram sums
+    const ScanColumn* cols;
+    const BColumn* bcols;
+    int has_cat, last_wins;
+    GainParamsDev gp;
+    LeafParams lp;
+    const uint8_t* colmask;  // [max_depth][n_cols], or null (column sampling)
+    const uint8_t* rmask;    // [n], or null (row sampling)
+    HBin* hist;              // [2^max_depth] slots (only the owning block touches a column)
+    uint64_t slot_bins;
+    ColCand* cand;           // [2^(max_depth - 1)][n_cols]
+    uint16_t* rt;            // [n] scratch: tree node of each row
+    long long* tot;          // [2^max_depth][2] scratch: node totals, level by level
+    // zero at launch:
+    uint32_t* bar;                 // grid barrier arrivals
+    unsigned long long* keys;      // [2^max_depth] best candidate per node
+    uint32_t *cnt, *scnt;          // [2^max_depth] rows / sampled rows per node
+    unsigned long long* xsum;      // [2^(max_depth + 1)][2] leaf sums
+    BState* state;                 // receives n_tnodes, hist_rows and err
+    BTreeNode* tree;
+    float* pred;
+    uint32_t* row_leaf;      // or null
+};
+// Whether a tree over n rows with columns of at most max_bins bins can be
+// grown that way on the current device.
+bool small_tree_fits(int mode, uint64_t n, uint32_t max_bins, bool has_cat);
+void launch_small_tree(const SmallTree& a, cudaStream_t st);
 
 // ---- K9 forest traversal ----------------------------------------------------
 // Node: word0 = feature | (is_leaf << 31) | (default_left << 30) | (categorical << 29)
