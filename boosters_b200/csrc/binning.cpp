@@ -203,14 +203,20 @@ bst_status plan_binning(const float* x, uint64_t F, uint64_t n,
     // the row sample (sequential draws) on one thread while the others
     // analyse the features
     std::vector<uint32_t> sample;
-    std::thread sampler([&] { sample = binning_sample(n, cfg.binning_sample_cnt); });
-#pragma omp parallel for schedule(dynamic, 1)
+    std::thread sampler;
+    if (n > cfg.binning_sample_cnt) sampler = std::thread([&] { sample = binning_sample(n, cfg.binning_sample_cnt); });
+    // A thread per 2^17 values, and some cores left to the sampler, the upload
+    // and the caller: a team as wide as the machine kept one of them waiting
+    // for a 4 ms time slice in half the calls.
+    const int64_t cores = omp_get_max_threads();
+    const int team = (int)std::max<int64_t>(1, std::min<int64_t>(cores * 3 / 4, (int64_t)(n * F >> 17)));
+#pragma omp parallel for schedule(dynamic, 1) num_threads(team)
     for (int64_t f = 0; f < (int64_t)F; ++f) {
         const float* col = x + (uint64_t)f * n;
         const bool uc = (size_t)f < user_cat.size() && user_cat[f];
         facts[f] = analyze(col, n, cfg, uc);
     }
-    sampler.join();
+    if (sampler.joinable()) sampler.join();
 
     // numeric features: bounds from the sampled values off the host, while
     // the host takes the categorical ones
@@ -223,11 +229,14 @@ bst_status plan_binning(const float* x, uint64_t F, uint64_t n,
         }
     if (!num_f.empty()) numeric.start(sample, num_f, num_nan, cfg.max_bins);
 
-#pragma omp parallel for schedule(dynamic, 1)
-    for (int64_t f = 0; f < (int64_t)F; ++f) {
+    std::vector<uint32_t> cat_f;
+    for (uint64_t f = 0; f < F; ++f)
+        if (!facts[f].trivial && !facts[f].numeric) cat_f.push_back((uint32_t)f);
+    const int cat_team = (int)std::max<int64_t>(1, std::min<int64_t>(team, (int64_t)cat_f.size()));
+#pragma omp parallel for schedule(dynamic, 1) num_threads(cat_team)
+    for (int64_t k = 0; k < (int64_t)cat_f.size(); ++k) {
+        const uint32_t f = cat_f[k];
         const float* col = x + (uint64_t)f * n;
-        const FeatureFacts& ff = facts[f];
-        if (ff.trivial || ff.numeric) continue;
         {
             // every finite value's category, not a sample (dataset.rs:655-672):
             // categories in [0, 65536) in a bitmap, any others in a hash set;

@@ -147,6 +147,7 @@ const char* bst_version(void) { return "boosters-b200 0.1.0 (sm_100a)"; }
 void bst_release_cached_memory(void) {
     bst::dev_cache_trim();
     bst::pinned_cache_trim();
+    bst::stream_pool_trim();
 }
 
 void bst_config_default(bst_config* c) {

@@ -160,6 +160,161 @@ void pinned_cache_trim() {
     c.bytes = 0;
 }
 
+// Idle streams of finished calls, kept per device for the next (creating and
+// destroying one costs 0.15 ms and more on a busy host).
+namespace {
+struct StreamPool {
+    std::mutex mu;
+    std::vector<std::pair<int, cudaStream_t>> idle;  // (device, stream)
+};
+StreamPool& stream_pool() {
+    static StreamPool* p = new StreamPool();  // never destroyed (see dev_cache)
+    return *p;
+}
+constexpr size_t STREAM_POOL_MAX = 16;
+
+struct StreamGuard {
+    cudaStream_t s = nullptr;
+    int dev = 0;
+    StreamGuard() {
+        BST_CK(cudaGetDevice(&dev));
+        StreamPool& p = stream_pool();
+        {
+            std::lock_guard<std::mutex> lk(p.mu);
+            for (size_t i = 0; i < p.idle.size(); ++i)
+                if (p.idle[i].first == dev) {
+                    s = p.idle[i].second;
+                    p.idle.erase(p.idle.begin() + i);
+                    return;
+                }
+        }
+        BST_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    }
+    StreamGuard(const StreamGuard&) = delete;
+    StreamGuard& operator=(const StreamGuard&) = delete;
+    ~StreamGuard() {
+        if (!s) return;
+        if (cudaStreamSynchronize(s) == cudaSuccess) {  // idle, and not left in a capture
+            StreamPool& p = stream_pool();
+            std::lock_guard<std::mutex> lk(p.mu);
+            if (p.idle.size() < STREAM_POOL_MAX) {
+                p.idle.emplace_back(dev, s);
+                return;
+            }
+        }
+        cudaGetLastError();
+        cudaStreamDestroy(s);
+    }
+};
+
+// A host array to the device in stream order. Pinned memory: one asynchronous
+// copy. Pageable memory: the driver's own staging runs at 11 GB/s on one
+// thread, so larger arrays go through pinned blocks filled by several threads
+// (120 MB: 10.5 -> 3.9 ms). finish(): the array has been read (the copies may
+// still run); the destructor waits for them.
+class HostUpload {
+  public:
+    HostUpload() = default;
+    HostUpload(const HostUpload&) = delete;
+    HostUpload& operator=(const HostUpload&) = delete;
+    ~HostUpload() {
+        join();
+        if (st_used_) cudaStreamSynchronize(st_);
+        for (auto& b : blocks_)
+            if (b.done) cudaEventDestroy(b.done);
+        pinned_free(pinned_);
+        cudaGetLastError();
+    }
+    void start(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+        if (!bytes) return;
+        cudaPointerAttributes a{};
+        const bool pinned = cudaPointerGetAttributes(&a, src) == cudaSuccess && a.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        if (pinned) {
+            BST_CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+            return;
+        }
+        BST_CK(cudaGetDevice(&dev_));
+        st_ = st;
+        dst_ = static_cast<char*>(dst);
+        src_ = static_cast<const char*>(src);
+        bytes_ = bytes;
+        size_t n = 1;
+        if (bytes >= MIN_STAGED) {
+            const size_t hw = std::max<size_t>(1, std::thread::hardware_concurrency());
+            n = std::max<size_t>(1, std::min<size_t>({MAX_THREADS, hw / 2, bytes / BLOCK}));
+        }
+        if (n > 1) {
+            blocks_.resize(2 * n);
+            pinned_ = static_cast<char*>(pinned_alloc(2 * n * BLOCK));
+            for (size_t i = 0; i < 2 * n; ++i) {
+                blocks_[i].p = pinned_ + i * BLOCK;
+                BST_CK(cudaEventCreateWithFlags(&blocks_[i].done, cudaEventDisableTiming));
+            }
+            st_used_ = true;
+            for (size_t t = 0; t < n; ++t) threads_.emplace_back([this, t] { stage(t); });
+        } else {
+            threads_.emplace_back([this] {  // such copies hold the calling thread
+                cudaError_t e = cudaSetDevice(dev_);
+                if (e == cudaSuccess) e = cudaMemcpyAsync(dst_, src_, bytes_, cudaMemcpyHostToDevice, st_);
+                if (e != cudaSuccess) err_ = (int)e;
+            });
+        }
+    }
+    void finish() {
+        join();
+        BST_CK((cudaError_t)err_.load());
+    }
+
+  private:
+    static constexpr size_t BLOCK = (size_t)1 << 20, MIN_STAGED = (size_t)4 << 20, MAX_THREADS = 6;
+    struct Block {
+        char* p = nullptr;
+        cudaEvent_t done = nullptr;
+    };
+    std::vector<Block> blocks_;  // two per thread
+    char* pinned_ = nullptr;
+    std::vector<std::thread> threads_;
+    std::atomic<size_t> next_{0};
+    std::atomic<int> err_{0};
+    cudaStream_t st_ = nullptr;
+    bool st_used_ = false;
+    int dev_ = 0;
+    char* dst_ = nullptr;
+    const char* src_ = nullptr;
+    size_t bytes_ = 0;
+
+    void join() {
+        for (auto& t : threads_)
+            if (t.joinable()) t.join();
+        threads_.clear();
+    }
+    void stage(size_t t) {
+        cudaError_t e = cudaSetDevice(dev_);
+        for (size_t k = 0; e == cudaSuccess && !err_; ++k) {
+            const size_t off = next_.fetch_add(1) * BLOCK;
+            if (off >= bytes_) break;
+            const size_t len = std::min(BLOCK, bytes_ - off);
+            Block& b = blocks_[2 * t + (k & 1)];
+            if (k > 1) e = cudaEventSynchronize(b.done);  // the block's copy two rounds ago
+            if (e != cudaSuccess) break;
+            std::memcpy(b.p, src_ + off, len);
+            e = cudaMemcpyAsync(dst_ + off, b.p, len, cudaMemcpyHostToDevice, st_);
+            if (e == cudaSuccess) e = cudaEventRecord(b.done, st_);
+        }
+        if (e != cudaSuccess) err_ = (int)e;
+    }
+};
+}  // namespace
+
+void stream_pool_trim() {
+    StreamPool& p = stream_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    for (auto& e : p.idle) cudaStreamDestroy(e.second);
+    cudaGetLastError();
+    p.idle.clear();
+}
+
 void dev_cache_trim() {
     DevCache& c = dev_cache();
     std::lock_guard<std::mutex> lk(c.mu);
@@ -346,6 +501,7 @@ void build_lane_tiles(const BinPlan& p, uint32_t max_bins, std::vector<LaneTile>
 
 namespace {
 
+constexpr double HIST_QUERY_BYTES = 1073741824.0;
 constexpr uint32_t PART_CHUNK_ROWS = 4096;
 constexpr uint32_t SUM_CHUNK_ROWS = 8192;
 
@@ -859,12 +1015,8 @@ class Trainer {
         const uint64_t nv = v.n;
         val_x_.alloc(std::max<uint64_t>(1, nv * v.F));
         if (nv * v.F) BST_CK(cudaMemcpy(val_x_.p, v.xdata(), sizeof(float) * nv * v.F, cudaMemcpyHostToDevice));
-        std::vector<float> init((size_t)G_ * nv);
-        for (uint32_t g = 0; g < G_; ++g)
-            std::fill(init.begin() + (size_t)g * nv, init.begin() + (size_t)(g + 1) * nv, m_.base[g]);
-        val_pred_.alloc(std::max<size_t>(1, init.size()));
-        if (!init.empty())
-            BST_CK(cudaMemcpy(val_pred_.p, init.data(), sizeof(float) * init.size(), cudaMemcpyHostToDevice));
+        val_pred_.alloc(std::max<size_t>(1, (size_t)G_ * nv));
+        for (uint32_t g = 0; g < G_; ++g) launch_fill_f32(val_pred_.p + (size_t)g * nv, m_.base[g], nv, st_);
     }
 
     // Metric of [G][n] raw margins on the device against labels y / weights
@@ -1159,9 +1311,7 @@ class Trainer {
             BST_CK(cudaMemcpy(alpha_.p, a.data(), sizeof(float) * G_, cudaMemcpyHostToDevice));
         }
         if (ds_.has_w) BST_CK(cudaMemcpyAsync(w_.p, ds_.w.data(), sizeof(float) * n, cudaMemcpyHostToDevice, st_));
-        std::vector<float> init((size_t)G_ * n);
-        for (uint32_t g = 0; g < G_; ++g) std::fill(init.begin() + (size_t)g * n, init.begin() + (size_t)(g + 1) * n, m_.base[g]);
-        BST_CK(cudaMemcpyAsync(pred_.p, init.data(), sizeof(float) * init.size(), cudaMemcpyHostToDevice, st_));
+        for (uint32_t g = 0; g < G_; ++g) launch_fill_f32(pred_.p + (size_t)g * n, m_.base[g], n, st_);
         BST_CK(cudaStreamSynchronize(st_));
     }
 
@@ -1176,9 +1326,11 @@ class Trainer {
         if (n_cols_) {
             // one histogram per partition node (the reference's LRU pool is
             // unnecessary with 180 GB of HBM); refuse sizes that cannot fit
-            size_t free_b = 0, total_b = 0;
-            BST_CK(cudaMemGetInfo(&free_b, &total_b));
+            // (the free memory is asked for only when they take a fair share
+            // of the device: the query takes 0.02 to 80 ms on a shared host)
             double need = (double)max_pnodes_ * (double)slot_bins_ * sizeof(HBin);
+            size_t free_b = std::numeric_limits<size_t>::max(), total_b = 0;
+            if (need > HIST_QUERY_BYTES) BST_CK(cudaMemGetInfo(&free_b, &total_b));
             if (leafwise_ && need > 0.6 * (double)free_b && max_pnodes_ > cfg_.max_leaves) {
                 max_pnodes_ = std::max<uint32_t>(1, cfg_.max_leaves);  // no room to speculate
                 need = (double)max_pnodes_ * (double)slot_bins_ * sizeof(HBin);
@@ -2837,14 +2989,6 @@ void base_scores(const HostDataset& ds, const bst_config& cfg, uint32_t G, std::
     }
 }
 
-struct StreamGuard {
-    cudaStream_t s = nullptr;
-    StreamGuard() { BST_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
-    ~StreamGuard() {
-        if (s) cudaStreamDestroy(s);
-    }
-};
-
 }  // namespace
 
 uint32_t n_outputs_of(const bst_config& c) {
@@ -2948,44 +3092,18 @@ void make_binned(const HostDataset& ds, const bst_config& cfg, cudaStream_t st, 
     BST_RANGE("bst.binning");
     std::string err;
     const auto t0 = std::chrono::steady_clock::now();
-    // Every feature goes to the device while the host analyses them: from
-    // pinned memory as one asynchronous copy, from pageable memory on a
-    // helper thread (such copies hold the calling thread). The numeric
-    // features' bounds are then computed on the device from that copy.
+    // Every feature goes to the device while the host analyses them; the
+    // numeric features' bounds are then computed on the device from that copy.
     DevArray<float> x;
-    std::thread uploader;
-    struct Joiner {
-        std::thread& t;
-        ~Joiner() {
-            if (t.joinable()) t.join();
-        }
-    } joiner{uploader};
-    cudaError_t up_err = cudaSuccess;
+    HostUpload up;
     if (ds.n && ds.F) {
         x.alloc((size_t)ds.F * ds.n);
-        cudaPointerAttributes a{};
-        const bool pinned = cudaPointerGetAttributes(&a, ds.xdata()) == cudaSuccess && a.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        const size_t bytes = sizeof(float) * ds.F * ds.n;
-        if (pinned) {
-            BST_CK(cudaMemcpyAsync(x.p, ds.xdata(), bytes, cudaMemcpyHostToDevice, st));
-        } else {
-            int dev = 0;
-            BST_CK(cudaGetDevice(&dev));
-            uploader = std::thread([&x, &ds, &up_err, bytes, dev, st] {
-                up_err = cudaSetDevice(dev);
-                if (up_err == cudaSuccess) up_err = cudaMemcpyAsync(x.p, ds.xdata(), bytes, cudaMemcpyHostToDevice, st);
-            });
-        }
+        up.start(x.p, ds.xdata(), sizeof(float) * ds.F * ds.n, st);
     }
-    DeviceBounds numeric(x.p, ds.n, st, [&] {
-        if (uploader.joinable()) uploader.join();
-        BST_CK(up_err);
-    });
+    DeviceBounds numeric(x.p, ds.n, st, [&] { up.finish(); });
     bst_status rc = plan_binning(ds.xdata(), ds.F, ds.n, ds.user_cat, cfg, numeric, out.plan, err);
     if (rc != BST_OK) throw Error{rc, err};
-    if (uploader.joinable()) uploader.join();
-    BST_CK(up_err);
+    up.finish();
     const BinPlan& p = out.plan;
     const uint32_t nc = p.n_cols();
     const uint64_t n = p.n;
@@ -3567,7 +3685,9 @@ void predict_host(const Model& m, const HostDataset& ds, bool raw, float* out) {
     DevArray<float> x, o;
     x.alloc((size_t)n * ds.F);
     o.alloc((size_t)n * m.n_groups);
-    BST_CK(cudaMemcpyAsync(x.p, ds.xdata(), sizeof(float) * n * ds.F, cudaMemcpyHostToDevice, sg.s));
+    HostUpload up;
+    up.start(x.p, ds.xdata(), sizeof(float) * n * ds.F, sg.s);
+    up.finish();
     // The shared-memory traversal where the forest has it and its bin tiles
     // fit in device memory, else the node list (one thread per row, every
     // node from L2): 300,000 x 100 rows through 500 trees of depth 8 take

@@ -48,7 +48,8 @@ void dev_cache_trim();  // frees every cached block
 // for the device to be idle, as cudaFreeHost does, then keeps the block).
 void* pinned_alloc(size_t bytes);
 void pinned_free(void* p);
-void pinned_cache_trim();  // frees every cached pinned block
+void pinned_cache_trim();
+void stream_pool_trim();  // frees every cached pinned block
 
 template <class T>
 struct DevArray {

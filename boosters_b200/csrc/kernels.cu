@@ -5073,6 +5073,17 @@ void launch_goss_apply(float2* gh, const uint8_t* code, float mult, uint8_t* mas
     launch_k(k_goss_apply, (unsigned)blocks, 256, 0, st, gh, code, mult, mask, n);
 }
 
+__global__ void k_fill_f32(float* __restrict__ a, float v, uint64_t n) {
+    BST_PDL_ENTER();
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) a[i] = v;
+}
+
+void launch_fill_f32(float* a, float v, uint64_t n, cudaStream_t st) {
+    if (n == 0) return;
+    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16);
+    launch_k(k_fill_f32, (unsigned)blocks, 256, 0, st, a, v, n);
+}
+
 __global__ void k_add_f32(float* __restrict__ a, const float* __restrict__ b, uint64_t n) {
     BST_PDL_ENTER();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
