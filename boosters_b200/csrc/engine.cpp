@@ -801,6 +801,77 @@ struct Cand {
     uint32_t count;
 };
 
+// Node lists of `trees` in forest order (ForestDev's arrays).
+struct NodeForest {
+    std::vector<ForestNode> nodes;
+    std::vector<uint32_t> roots, cat_seg, cat_words, group_trees, group_off;
+};
+NodeForest node_forest(const std::vector<const HostTree*>& trees, uint32_t n_groups) {
+    NodeForest f;
+    for (const HostTree* tp : trees) {
+        const HostTree& t = *tp;
+        const uint32_t base_idx = (uint32_t)f.nodes.size();
+        const uint32_t wbase = (uint32_t)f.cat_words.size();
+        f.roots.push_back(base_idx);
+        for (size_t i = 0; i < t.split_index.size(); ++i) {
+            ForestNode fn;
+            fn.word = (t.split_index[i] & 0x1FFFFFFFu) | ((uint32_t)t.is_leaf[i] << 31) |
+                      ((uint32_t)t.default_left[i] << 30) | ((uint32_t)(t.split_type[i] == 1) << 29);
+            fn.value = t.is_leaf[i] ? t.leaf[i] : t.threshold[i];
+            fn.left = base_idx + t.left[i];
+            fn.right = base_idx + t.right[i];
+            f.nodes.push_back(fn);
+            const uint32_t ss = t.seg_size.empty() ? 0 : t.seg_size[i];
+            f.cat_seg.push_back(ss ? wbase + t.seg_start[i] : 0);
+            f.cat_seg.push_back(ss);
+        }
+        f.cat_words.insert(f.cat_words.end(), t.cat_words.begin(), t.cat_words.end());
+    }
+    f.group_off.assign(n_groups + 1, 0);
+    for (uint32_t g = 0; g < n_groups; ++g) {
+        f.group_off[g] = (uint32_t)f.group_trees.size();
+        for (uint32_t t = 0; t < trees.size(); ++t)
+            if (trees[t]->group == g) f.group_trees.push_back(t);
+    }
+    f.group_off[n_groups] = (uint32_t)f.group_trees.size();
+    return f;
+}
+
+// The trees of one round on the device: one buffer, grown as needed and
+// reused, one copy in stream order.
+struct RoundForest {
+    DevArray<char> dev;
+    std::vector<char> host;
+    ForestDev view{};
+    void upload(const std::vector<const HostTree*>& trees, uint32_t n_groups, cudaStream_t st) {
+        const NodeForest f = node_forest(trees, n_groups);
+        host.clear();
+        auto put = [&](const auto& v) {  // 16-byte aligned
+            const size_t at = host.size(), bytes = sizeof(v[0]) * v.size();
+            host.resize(at + (bytes + 15) / 16 * 16);
+            if (bytes) std::memcpy(host.data() + at, v.data(), bytes);
+            return at;
+        };
+        const size_t o[6] = {put(f.nodes),   put(f.roots),     put(f.group_trees),
+                             put(f.group_off), put(f.cat_seg), put(f.cat_words)};
+        if (dev.n < host.size()) dev.alloc(2 * host.size());
+        BST_CK(cudaMemcpyAsync(dev.p, host.data(), host.size(), cudaMemcpyHostToDevice, st));
+        auto at = [&](int k) { return reinterpret_cast<const uint32_t*>(dev.p + o[k]); };
+        view.nodes = reinterpret_cast<const ForestNode*>(dev.p);
+        view.roots = at(1);
+        view.group_trees = at(2);
+        view.group_off = at(3);
+        view.cat_seg = at(4);
+        view.cat_words = at(5);
+        view.base = nullptr;  // not read by the evaluation
+        view.n_trees = (uint32_t)trees.size();
+        view.n_groups = n_groups;
+#ifdef BST_CHECKED
+        view.chk_nodes = (uint32_t)f.nodes.size();
+#endif
+    }
+};
+
 class Trainer {
   public:
     Trainer(const HostDataset& ds, const DeviceBinned& b, const bst_config& cfg, uint32_t n_threads,
@@ -1006,39 +1077,84 @@ class Trainer {
     }
 
     // ---- early-stopping evaluation -------------------------------------------
+    static_assert(EVAL_RMSE == BST_METRIC_RMSE && EVAL_LOGLOSS == BST_METRIC_LOGLOSS &&
+                      EVAL_MLOGLOSS == BST_METRIC_MLOGLOSS && EVAL_MAE == BST_METRIC_MAE && EVAL_MAPE == BST_METRIC_MAPE &&
+                      EVAL_QUANTILE == BST_METRIC_QUANTILE && EVAL_HUBER == BST_METRIC_HUBER &&
+                      EVAL_POISSON == BST_METRIC_POISSON && EVAL_MARGIN_ACCURACY == BST_METRIC_MARGIN_ACCURACY,
+                  "metric codes");
     const HostDataset* val_ = nullptr;
-    DevArray<float> val_x_, val_pred_, eval_tmp_;
-    std::vector<float> eval_host_;
+    DevArray<float> val_x_, val_y_, val_w_, val_pred_, eval_alpha_;
+    DevArray<double> eval_partial_;
+    std::vector<double> eval_host_;
+    RoundForest eval_forest_;  // the round's trees (one buffer, reused)
 
     void setup_validation(const HostDataset& v) {
         val_ = &v;
         const uint64_t nv = v.n;
         val_x_.alloc(std::max<uint64_t>(1, nv * v.F));
-        if (nv * v.F) BST_CK(cudaMemcpy(val_x_.p, v.xdata(), sizeof(float) * nv * v.F, cudaMemcpyHostToDevice));
+        HostUpload up;
+        up.start(val_x_.p, v.xdata(), sizeof(float) * nv * v.F, st_);
+        val_y_.alloc(std::max<uint64_t>(1, nv));
+        if (nv) BST_CK(cudaMemcpyAsync(val_y_.p, v.y.data(), sizeof(float) * nv, cudaMemcpyHostToDevice, st_));
+        if (v.has_w) {
+            val_w_.alloc(std::max<uint64_t>(1, nv));
+            if (nv) BST_CK(cudaMemcpyAsync(val_w_.p, v.w.data(), sizeof(float) * nv, cudaMemcpyHostToDevice, st_));
+        }
         val_pred_.alloc(std::max<size_t>(1, (size_t)G_ * nv));
         for (uint32_t g = 0; g < G_; ++g) launch_fill_f32(val_pred_.p + (size_t)g * nv, m_.base[g], nv, st_);
+        up.finish();
     }
 
-    // Metric of [G][n] raw margins on the device against labels y / weights
-    // w (host): transformed copy (Evaluator::compute, eval.rs:150-185), read
-    // back, summed on the host.
-    double device_metric(int metric, const float* margins, uint64_t n, const float* y, const float* w) {
-        const size_t cnt = (size_t)G_ * n;
-        if (cnt == 0) return 0.0;
-        eval_tmp_.alloc(cnt);
-        BST_CK(cudaMemcpyAsync(eval_tmp_.p, margins, sizeof(float) * cnt, cudaMemcpyDeviceToDevice, st_));
+    // The metric of the margins in `a` (every row summed on the device in
+    // f64; the outputs' sums finished here), after the round's trees.
+    double evaluate(EvalArgs a, int metric) {
+        if (a.n == 0) return 0.0;
+        const MetricParams mp = metric_params(cfg_);
+        a.G = G_;
+        a.metric = metric;
         // every metric but the margin accuracy reads transformed predictions
         // (eval.rs:151, metrics/mod.rs:272-286)
-        if (metric != BST_METRIC_MARGIN_ACCURACY)
-            launch_transform(transform_of(cfg_.objective), eval_tmp_.p, G_, n, st_);
-        eval_host_.resize(cnt);
-        BST_CK(cudaMemcpyAsync(eval_host_.data(), eval_tmp_.p, sizeof(float) * cnt, cudaMemcpyDeviceToHost, st_));
+        a.transform = transform_of(cfg_.objective);
+        a.delta = mp.delta;
+        a.n_alpha = mp.alpha ? mp.n_alpha : 0u;
+        eval_alpha_.alloc(std::max<uint32_t>(1, a.n_alpha));
+        if (a.n_alpha && eval_host_.empty())
+            BST_CK(cudaMemcpy(eval_alpha_.p, mp.alpha, sizeof(float) * a.n_alpha, cudaMemcpyHostToDevice));
+        a.alpha = eval_alpha_.p;
+        const uint32_t outs = metric == BST_METRIC_MAE || metric == BST_METRIC_RMSE || metric == BST_METRIC_QUANTILE ? G_ : 1u;
+        const uint32_t blocks = eval_blocks(a.n);
+        eval_partial_.alloc((size_t)blocks * outs * 2);
+        eval_host_.resize((size_t)blocks * outs * 2);
+        a.partial = eval_partial_.p;
+        launch_evaluate(a, st_);
+        BST_CK(cudaGetLastError());
+        BST_CK(cudaMemcpyAsync(eval_host_.data(), eval_partial_.p, sizeof(double) * eval_host_.size(),
+                               cudaMemcpyDeviceToHost, st_));
         BST_CK(cudaStreamSynchronize(st_));
-        return metric_value(metric, eval_host_.data(), G_, n, y, w, metric_params(cfg_));
+        double sum = 0.0, tl = 0.0, tw = 0.0;
+        for (uint32_t o = 0; o < outs; ++o) {
+            double t = 0.0, w = 0.0;
+            for (uint32_t b = 0; b < blocks; ++b) {
+                t += eval_host_[((size_t)b * outs + o) * 2];
+                w += eval_host_[((size_t)b * outs + o) * 2 + 1];
+            }
+            tl += t;
+            tw += w;
+            const double mean = w > 0.0 ? t / w : 0.0;
+            sum += metric == BST_METRIC_RMSE ? (w > 0.0 ? std::sqrt(mean) : 0.0) : mean;
+        }
+        if (metric == BST_METRIC_QUANTILE) return tw > 0.0 ? tl / tw : 0.0;
+        if (metric == BST_METRIC_MAPE) return sum * 100.0;
+        return sum / (double)outs;
     }
 
     double train_value(int metric) {
-        return device_metric(metric, pred_.p, n_, ds_.y.data(), ds_.has_w ? ds_.w.data() : nullptr);
+        EvalArgs a{};
+        a.n = n_;
+        a.margins = pred_.p;
+        a.y = y_.p;
+        a.w = ds_.has_w ? w_.p : nullptr;
+        return evaluate(a, metric);
     }
 
     // Adds the trees pushed since `first` (this round's, one per output) to
@@ -1046,18 +1162,20 @@ class Trainer {
     // then the validation metric.
     double validation_value(int metric, size_t first) {
         const HostDataset& v = *val_;
+        EvalArgs a{};
+        a.n = v.n;
         if (v.n && m_.trees.size() > first) {
             std::vector<const HostTree*> tp;
             for (size_t t = first; t < m_.trees.size(); ++t) tp.push_back(&m_.trees[t]);
-            DeviceForest f;
-            upload_node_forest(tp, G_, std::vector<float>(G_, 0.0f), f);
-            eval_tmp_.alloc((size_t)G_ * v.n);
-            launch_predict(f.view, val_x_.p, v.n, (uint32_t)v.F, 1, eval_tmp_.p, st_);
-            launch_add_f32(val_pred_.p, eval_tmp_.p, (uint64_t)G_ * v.n, st_);
-            BST_CK(cudaGetLastError());
-            BST_CK(cudaStreamSynchronize(st_));  // f is freed on return
+            eval_forest_.upload(tp, G_, st_);
+            a.forest = eval_forest_.view;
         }
-        return device_metric(metric, val_pred_.p, v.n, v.y.data(), v.has_w ? v.w.data() : nullptr);
+        a.x = val_x_.p;
+        a.n_features = (uint32_t)v.F;
+        a.margins = val_pred_.p;
+        a.y = val_y_.p;
+        a.w = v.has_w ? val_w_.p : nullptr;
+        return evaluate(a, metric);
     }
 
     // Training predictions back to the model.
@@ -3266,44 +3384,18 @@ std::unique_ptr<Model> Booster::snapshot() const {
 void upload_node_forest(const std::vector<const HostTree*>& trees, uint32_t n_groups, const std::vector<float>& base,
                         DeviceForest& df) {
     DeviceForest* f = &df;
-    std::vector<ForestNode> nodes;
-    std::vector<uint32_t> roots, cat_seg, cat_words, gt, goff(n_groups + 1, 0);
-    for (const HostTree* tp : trees) {
-        const HostTree& t = *tp;
-        const uint32_t base_idx = (uint32_t)nodes.size();
-        const uint32_t wbase = (uint32_t)cat_words.size();
-        roots.push_back(base_idx);
-        for (size_t i = 0; i < t.split_index.size(); ++i) {
-            ForestNode fn;
-            fn.word = (t.split_index[i] & 0x1FFFFFFFu) | ((uint32_t)t.is_leaf[i] << 31) |
-                      ((uint32_t)t.default_left[i] << 30) | ((uint32_t)(t.split_type[i] == 1) << 29);
-            fn.value = t.is_leaf[i] ? t.leaf[i] : t.threshold[i];
-            fn.left = base_idx + t.left[i];
-            fn.right = base_idx + t.right[i];
-            nodes.push_back(fn);
-            const uint32_t ss = t.seg_size.empty() ? 0 : t.seg_size[i];
-            cat_seg.push_back(ss ? wbase + t.seg_start[i] : 0);
-            cat_seg.push_back(ss);
-        }
-        cat_words.insert(cat_words.end(), t.cat_words.begin(), t.cat_words.end());
-    }
-    for (uint32_t g = 0; g < n_groups; ++g) {
-        goff[g] = (uint32_t)gt.size();
-        for (uint32_t t = 0; t < trees.size(); ++t)
-            if (trees[t]->group == g) gt.push_back(t);
-    }
-    goff[n_groups] = (uint32_t)gt.size();
+    const NodeForest nf = node_forest(trees, n_groups);
     auto up = [](auto& dst, const auto& src) {
         dst.alloc(std::max<size_t>(1, src.size()));
         if (!src.empty())
             BST_CK(cudaMemcpy(dst.p, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice));
     };
-    up(f->nodes, nodes);
-    up(f->roots, roots);
-    up(f->group_trees, gt);
-    up(f->group_off, goff);
-    up(f->cat_seg, cat_seg);
-    up(f->cat_words, cat_words);
+    up(f->nodes, nf.nodes);
+    up(f->roots, nf.roots);
+    up(f->group_trees, nf.group_trees);
+    up(f->group_off, nf.group_off);
+    up(f->cat_seg, nf.cat_seg);
+    up(f->cat_words, nf.cat_words);
     up(f->base, base);
     f->view.nodes = f->nodes.p;
     f->view.roots = f->roots.p;
@@ -3315,7 +3407,7 @@ void upload_node_forest(const std::vector<const HostTree*>& trees, uint32_t n_gr
     f->view.n_trees = (uint32_t)trees.size();
     f->view.n_groups = n_groups;
 #ifdef BST_CHECKED
-    f->view.chk_nodes = (uint32_t)nodes.size();
+    f->view.chk_nodes = (uint32_t)nf.nodes.size();
 #endif
 }
 

@@ -659,8 +659,27 @@ void launch_predict_heap(const HeapForest& f, const float* x, uint64_t n, uint32
 void launch_transform(int transform, float* out, uint32_t G, uint64_t n, cudaStream_t st);
 // a[i] = v, i < n
 void launch_fill_f32(float* a, float v, uint64_t n, cudaStream_t st);
-// a[i] = a[i] + b[i] (f32), i < n
-void launch_add_f32(float* a, const float* b, uint64_t n, cudaStream_t st);
+// Metrics (values = BST_METRIC_*) and one round's evaluation on the device.
+enum EvalMetric : int {
+    EVAL_RMSE = 1, EVAL_LOGLOSS, EVAL_MLOGLOSS, EVAL_MAE, EVAL_MAPE, EVAL_QUANTILE, EVAL_HUBER, EVAL_POISSON,
+    EVAL_MARGIN_ACCURACY
+};
+struct EvalArgs {
+    ForestDev forest;   // the round's trees (n_trees 0: none)
+    const float* x;     // [n_features][n], read by the trees
+    uint32_t n_features, G;
+    uint64_t n;
+    float* margins;     // [G][n] raw margins, the trees' leaves added
+    const float* y;     // [n]
+    const float* w;     // [n] or null
+    const float* alpha; // quantile: [n_alpha]
+    uint32_t n_alpha;
+    float delta;        // Huber
+    int transform, metric;
+    double* partial;    // [eval_blocks(n)][outputs][2]: weighted sum, weight
+};
+uint32_t eval_blocks(uint64_t n);
+void launch_evaluate(const EvalArgs& a, cudaStream_t st);
 // gh[i] = (0, 0) where mask[i] == 0 (row sampling), i < n
 void launch_zero_unsampled(float2* gh, const uint8_t* mask, uint64_t n, cudaStream_t st);
 // GOSS codes (0 out, 1 kept, 2 kept and scaled by mult) applied to one
