@@ -1918,6 +1918,93 @@ __device__ __forceinline__ uint32_t sat_sub(uint32_t a, uint32_t b) { return a >
 
 constexpr int SCAN_WARPS = 8;
 constexpr int SORT_N = 256;  // categorical columns with <= 256 bins
+constexpr int SCAN_PER = 9;  // consecutive bins per lane of a numeric column's search: up to 288 bins
+
+// Shared scratch of a warp's search: the bins of a numeric column, or a
+// categorical column's sort keys (f64) and categories.
+template <typename HB>
+__host__ __device__ constexpr uint32_t scan_scratch() {
+    return (uint32_t)(32 * SCAN_PER * sizeof(HB) > SORT_N * 12 ? 32 * SCAN_PER * sizeof(HB) : SORT_N * 12);
+}
+
+// Sums of hessians from h on pass `(double)h * ih >= mcw`, none below do (the
+// product is monotone in h); exact: h is known (else the test itself is made).
+struct HessMin {
+    long long h;
+    bool exact;
+};
+__device__ __forceinline__ HessMin hess_min(double mcw, double ih) {
+    HessMin r{0, false};
+    const double h0 = mcw / ih;
+    if (!(fabs(h0) < 1.0e15)) return r;
+    r.h = (long long)ceil(h0);
+    if ((double)(r.h - 1) * ih >= mcw)
+        --r.h;
+    else if (!((double)r.h * ih >= mcw))
+        ++r.h;
+    r.exact = (double)r.h * ih >= mcw && !((double)(r.h - 1) * ih >= mcw);
+    return r;
+}
+
+// Lambda in units of the hessian sums; out of range: -infinity (no filter).
+__device__ __forceinline__ float hess_lambda(double lambda, double ih) {
+    const double l = lambda / ih;
+    return l >= 0.0 && l < 1.0e36 ? (float)l : -INFINITY;
+}
+
+// Units of the histogram sums and what follows from them, once per warp.
+struct ScanUnits {
+    double ig, ih;
+    HessMin hmin;
+    float lam;
+    __device__ ScanUnits(const double* scale, const GainParamsDev& gp)
+        : ig(scale[2]), ih(scale[3]), hmin(hess_min(gp.min_child_weight, scale[3])), lam(hess_lambda(gp.lambda, scale[3])) {}
+};
+
+// Largest approximate score gl^2 / (hl + lambda) + gr^2 / (hr + lambda), in
+// units of the integer sums, of the valid candidates at bin b (forward, and
+// backward when the column has a missing bin; find.rs:286-407): -1 when there
+// is none, infinity when it cannot be bounded. P: the bins' sums up to b, T:
+// the node's totals, M: the totals without the last (missing) bin. The f32
+// score is off by less than 2^-19 of itself.
+template <typename Acc>
+struct ScoreRule {  // one node's
+    Acc hmin;
+    uint32_t msl, most;  // a candidate's bin count is in [msl, most] (sat_sub(pc, count) >= msl)
+    float lam;
+    bool safe;  // every valid candidate has positive denominators
+    double mcw, ih;
+    __device__ ScoreRule(const HessMin& m, float lam_, const GainParamsDev& gp, double ih_, uint32_t pc)
+        : hmin((Acc)m.h),
+          msl(gp.min_samples_leaf),
+          most(gp.min_samples_leaf == 0 ? 0xFFFFFFFFu : sat_sub(pc, gp.min_samples_leaf)),
+          lam(lam_),
+          safe(m.exact && (long long)(Acc)m.h == m.h && m.h >= 0 && lam_ >= 0.0f && (m.h >= 1 || lam_ > 0.0f)),
+          mcw(gp.min_child_weight),
+          ih(ih_) {}
+    __device__ __forceinline__ float one(Acc lg, Acc lh, Acc rg, Acc rh, uint32_t count) const {
+        if (count < msl || count > most) return -1.0f;
+        if (!safe) return (double)lh * ih >= mcw && (double)rh * ih >= mcw ? INFINITY : -1.0f;
+        if (lh < hmin || rh < hmin) return -1.0f;
+        const float gl = (float)lg, gr = (float)rg;
+        return gl * gl * rcp_approx((float)lh + lam) + gr * gr * rcp_approx((float)rh + lam);
+    }
+    static __device__ __forceinline__ float rcp_approx(float x) {  // within 1 ulp
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+        return r;
+    }
+    template <typename T2>
+    __device__ __forceinline__ float best(T2 P, T2 T, T2 M, uint32_t b, uint32_t nb, bool hm) const {
+        float s = -1.0f;
+        if (b + 1 < nb) s = one(P.x, P.y, T.x - P.x, T.y - P.y, b + 1);
+        if (hm && b + 2 < nb) {
+            const Acc Rg = M.x - P.x, Rh = M.y - P.y;
+            s = fmaxf(s, one(T.x - Rg, T.y - Rh, Rg, Rh, nb - 2 - b));
+        }
+        return s;
+    }
+};
 
 }  // namespace
 
@@ -2140,19 +2227,152 @@ __device__ __forceinline__ float scan_column(Ld ld, const ScanNode& nd, const Sc
     return best.gain;
 }
 
-// The same for column `col` of node `node`, whose histogram lives in slot
-// nd.slot: cand[node * n_cols + col] and, for column 0, the node totals.
-// cmask (or null): the node's column mask.
+// One warp: the same for a numeric column of up to 32 SCAN_PER bins at h. The
+// bins are read coalesced and passed through shared memory so that a lane
+// holds SCAN_PER consecutive ones (an odd stride: no bank conflicts): its
+// prefix sums are serial adds and one scan over the lanes, instead of one per
+// 32 bins. Every bin's score is bounded in f32 first; candidates whose score
+// is within 2^-16 of the column's best get their exact gain (the gain is half
+// the score less an offset >= 0, so no other can win or tie; without a bound
+// all do), so the f64 divisions run once or twice per column and warp instead
+// of 8 to 16 times. 1M x 100, depth 8: the searches of a q8 tree 130 us, before
+// 158; of an fp32 tree 156, before 175; a level of few nodes 11.5, before 14
+// (half of it the hand-off to the last block and its decisions).
 template <typename HB>
-__device__ float scan_item(const ScanNode nd, uint32_t node, uint32_t col, const ScanColumn* __restrict__ cols,
-                          uint32_t n_cols, const HB* __restrict__ hist, uint64_t slot_bins,
-                          const double* __restrict__ scale, const GainParamsDev& gp, ColCand* __restrict__ cand,
-                          long long* __restrict__ node_tot, double* key, uint32_t* cat,
-                          const uint8_t* __restrict__ cmask) {
-    const ScanColumn cm = cols[col];
+__device__ __forceinline__ float scan_numeric(const HB* h, const ScanNode& nd, const ScanColumn& cm, const ScanUnits& un,
+                                              const GainParamsDev& gp, ColCand* out, long long* tot, HB* buf,
+                                              bool masked) {
+    using Acc = decltype(HB{}.g);
+    struct alignas(sizeof(HB)) T2 {
+        Acc x, y;
+    };
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t nb = cm.n_bins, pc = nd.count;
+    T2* row = reinterpret_cast<T2*>(buf);
+    {
+        T2 v[SCAN_PER];
+#pragma unroll
+        for (uint32_t q = 0; q < SCAN_PER; ++q) {
+            const uint32_t b = q * 32u + lane;
+            v[q].x = v[q].y = 0;
+            if (b < nb) v[q] = reinterpret_cast<const T2*>(h)[b];
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < SCAN_PER; ++q) row[q * 32u + lane] = v[q];
+    }
+    const double ig = un.ig, ih = un.ih;
+    __syncwarp();
+    T2 P[SCAN_PER];
+    Acc sg = 0, sh = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < SCAN_PER; ++k) {
+        const T2 v = row[lane * SCAN_PER + k];
+        sg += v.x;
+        sh += v.y;
+        P[k].x = sg;
+        P[k].y = sh;
+    }
+    const T2 last = row[nb - 1];
+    const Acc ig_ = warp_incl_scan(sg, (int)lane), ih_ = warp_incl_scan(sh, (int)lane);
+    T2 T;
+    T.x = __shfl_sync(FULL, ig_, 31);
+    T.y = __shfl_sync(FULL, ih_, 31);
+    const Acc eg = ig_ - sg, eh = ih_ - sh;
+    if (nd.flags & 1u) {  // explicit node totals
+        T.x = (Acc)nd.pg;
+        T.y = (Acc)nd.ph;
+    }
+    if (tot && lane == 0) {
+        tot[0] = T.x;
+        tot[1] = T.y;
+    }
+    __syncwarp();
+    Best best{-INFINITY, 0xFFFFFFFFu, 0u, 0u};
+    if (!masked && nb >= 2) {
+        T2 M;
+        M.x = T.x - last.x;
+        M.y = T.y - last.y;
+        const bool hm = cm.has_missing != 0;
+        const ScoreRule<Acc> rule(un.hmin, un.lam, gp, ih, pc);
+        float sc[SCAN_PER], mx = -1.0f;
+#pragma unroll
+        for (uint32_t k = 0; k < SCAN_PER; ++k) {
+            P[k].x += eg;
+            P[k].y += eh;
+            row[lane * SCAN_PER + k] = P[k];
+            sc[k] = rule.best(P[k], T, M, lane * SCAN_PER + k, nb, hm);
+            mx = fmaxf(mx, sc[k]);
+        }
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
+        if (mx >= 0.0f) {
+            // the offset's sign is known when the node's hessians are positive
+            const bool filter = mx < INFINITY && gp.min_gain >= 0.0 && T.y >= 0 && (float)T.y + un.lam > 0.0f;
+            const float thr = filter ? mx * (1.0f - 1.0f / 65536.0f) : 0.0f;
+            uint32_t todo = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < SCAN_PER; ++k) todo |= sc[k] >= thr ? 1u << k : 0u;
+            const double pg = (double)T.x * ig, ph = (double)T.y * ih;
+            GainCtx ctx;
+            ctx.lambda = gp.lambda;
+            ctx.offset = 0.5 * (pg * pg / (ph + gp.lambda)) + gp.min_gain;
+            ctx.mcw = gp.min_child_weight;
+            ctx.msl = gp.min_samples_leaf;
+            while (todo) {  // ascending bins
+                const uint32_t k = (uint32_t)__ffs((int)todo) - 1u, b = lane * SCAN_PER + k;
+                todo &= todo - 1u;
+                const T2 p = row[b];
+                if (b + 1 < nb) {  // forward candidate: bins <= b go left
+                    const double lg = (double)p.x * ig, lh = (double)p.y * ih;
+                    const double rg = (double)(T.x - p.x) * ig, rh = (double)(T.y - p.y) * ih;
+                    const uint32_t lc = b + 1, rc = sat_sub(pc, lc);
+                    if (ctx.valid(lh, rh, lc, rc)) {
+                        const float g = ctx.gain(lg, lh, rg, rh);
+                        if (better(g, b, best.gain, best.order)) best = Best{g, b, b, 0u};
+                    }
+                }
+                if (hm && b + 2 < nb) {  // backward candidate: bins b+1..nb-2 go right
+                    const Acc Rg = M.x - p.x, Rh = M.y - p.y;
+                    const double rg = (double)Rg * ig, rh = (double)Rh * ih;
+                    const double lg = (double)(T.x - Rg) * ig, lh = (double)(T.y - Rh) * ih;
+                    const uint32_t rc = nb - 2 - b, lc = sat_sub(pc, rc);
+                    if (ctx.valid(lh, rh, lc, rc)) {
+                        const float g = ctx.gain(lg, lh, rg, rh);
+                        const uint32_t ord = 2 * nb - 3 - b;
+                        if (better(g, ord, best.gain, best.order)) best = Best{g, ord, b, 1u};
+                    }
+                }
+            }
+            best = warp_best(best);
+        }
+    }
+    __syncwarp();  // the scratch is free for the warp's next column
+    if (lane == 0) {
+        out->gain = best.gain;
+        out->order = best.order;
+        out->bin = best.bin;
+        out->flags = best.flags;
+        out->cats[0] = out->cats[1] = out->cats[2] = out->cats[3] = 0ull;
+    }
+    return best.gain;
+}
+
+// One warp: best split of column `col` (facts cm) of node `node`, whose
+// histogram lives in slot nd.slot: cand[node * n_cols + col] and, for column
+// 0, the node totals. cmask (or null): the node's column mask. scratch: this
+// warp's scan_scratch<HB>() bytes.
+template <typename HB>
+__device__ float scan_item(const ScanNode& nd, const ScanColumn& cm, uint32_t node, uint32_t col, uint32_t n_cols,
+                           const HB* __restrict__ hist, uint64_t slot_bins, const double* __restrict__ scale,
+                           const ScanUnits& un, const GainParamsDev& gp, ColCand* __restrict__ cand,
+                           long long* __restrict__ node_tot, unsigned char* scratch, const uint8_t* __restrict__ cmask) {
     const HB* h = hist + (size_t)nd.slot * slot_bins + cm.hist_off;
-    return scan_column<HB>([h](uint32_t b) { return h[b]; }, nd, cm, scale, gp, cand + (size_t)node * n_cols + col,
-                           col == 0 ? node_tot + 2 * node : nullptr, key, cat, cmask && !cmask[col]);
+    ColCand* out = cand + (size_t)node * n_cols + col;
+    long long* tot = col == 0 ? node_tot + 2 * node : nullptr;
+    const bool masked = cmask && !cmask[col];
+    if (!cm.is_cat && cm.n_bins <= 32u * SCAN_PER && cm.n_bins)
+        return scan_numeric<HB>(h, nd, cm, un, gp, out, tot, reinterpret_cast<HB*>(scratch), masked);
+    return scan_column<HB>([h](uint32_t b) { return h[b]; }, nd, cm, scale, gp, out, tot,
+                           reinterpret_cast<double*>(scratch), reinterpret_cast<uint32_t*>(scratch + SORT_N * 8), masked);
 }
 
 template <typename HB>
@@ -2162,15 +2382,14 @@ k_split_scan(const ScanNode* __restrict__ nodes, const ScanColumn* __restrict__ 
              const double* __restrict__ scale, GainParamsDev gp, ColCand* __restrict__ cand,
              long long* __restrict__ node_tot, uint32_t col_blocks, const uint8_t* __restrict__ colmask) {
     BST_PDL_ENTER();
-    __shared__ double s_key[SCAN_WARPS][SORT_N];
-    __shared__ uint32_t s_cat[SCAN_WARPS][SORT_N];
+    __shared__ __align__(16) unsigned char scratch[SCAN_WARPS][scan_scratch<HB>()];
     const int warp = threadIdx.x >> 5;
     const uint32_t col = (blockIdx.x % col_blocks) * SCAN_WARPS + warp;
     const uint32_t node = blockIdx.x / col_blocks;
     if (col >= n_cols) return;
     const ScanNode nd = nodes[node];
-    scan_item(nd, node, col, cols, n_cols, hist, slot_bins, scale, gp, cand, node_tot, s_key[warp], s_cat[warp],
-              colmask ? colmask + (size_t)nd.pad * n_cols : nullptr);
+    scan_item(nd, cols[col], node, col, n_cols, hist, slot_bins, scale, ScanUnits(scale, gp), gp, cand, node_tot,
+              scratch[warp], colmask ? colmask + (size_t)nd.pad * n_cols : nullptr);
 }
 
 void launch_split_scan(const ScanNode* nodes, uint32_t n_nodes, const ScanColumn* cols,
@@ -2557,6 +2776,42 @@ __device__ uint32_t block_excl_scan(uint32_t v, uint32_t* sh, uint32_t* total) {
     return r;
 }
 
+// Two exclusive scans at once (sh: 66 words); synchronises like
+// block_excl_scan.
+__device__ void block_excl_scan2(uint32_t v, uint32_t w, uint32_t* sh, uint32_t* ev, uint32_t* ew, uint32_t* tv,
+                                 uint32_t* tw) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nw = (blockDim.x + 31) >> 5;
+    uint32_t x = v, y = w;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(FULL, x, d), u = __shfl_up_sync(FULL, y, d);
+        if (lane >= d) {
+            x += t;
+            y += u;
+        }
+    }
+    if (lane == 31) {
+        sh[warp] = x;
+        sh[33 + warp] = y;
+    }
+    __syncthreads();
+    uint32_t bx = 0, by = 0, ax = 0, ay = 0;  // sums of the warps before, of all
+    for (int q = 0; q < nw; ++q) {
+        const uint32_t t = sh[q], u = sh[33 + q];
+        if (q < warp) {
+            bx += t;
+            by += u;
+        }
+        ax += t;
+        ay += u;
+    }
+    *ev = bx + x - v;
+    *ew = by + y - w;
+    *tv = ax;
+    *tw = ay;
+    __syncthreads();
+}
+
 // GainParams::compute_leaf_weight (gain.rs:151-168) x learning rate (mutable_tree.rs:258).
 __device__ float leaf_value_dev(long long G, long long H, const double* scale, const LeafParams& lp) {
     const double g = (double)G * scale[2], h = (double)H * scale[3];
@@ -2666,7 +2921,7 @@ void launch_b_root_init(const BDev& d, uint32_t* ridx, uint64_t n, uint32_t chun
 constexpr uint32_t DECIDE_THREADS = SCAN_WARPS * 32;  // the block size of its one caller, k_b_scan
 
 __device__ void decide_body(BDev d, int a, LeafParams lp, const double* __restrict__ scale, uint32_t buf) {
-    __shared__ uint32_t sh[33];
+    __shared__ uint32_t sh[66];
     __shared__ uint32_t s_jc[DECIDE_THREADS], s_j[DECIDE_THREADS], s_begin[DECIDE_THREADS];
     __shared__ uint32_t base_exp, base_leaf, base_chunk, first_right, tn0, nf;
     BState* s = d.state;
@@ -2687,11 +2942,10 @@ __device__ void decide_body(BDev d, int a, LeafParams lp, const double* __restri
         if (valid) nd = A[i];
         const bool ex = valid && (nd.split.flags & 4u) && nd.split.gain > -INFINITY &&
                         !((double)nd.split.gain <= lp.min_gain);
-        uint32_t te, tl, tc;
-        const uint32_t je = block_excl_scan(ex ? 1u : 0u, sh, &te);
-        const uint32_t jl = block_excl_scan((valid && !ex) ? 1u : 0u, sh, &tl);
         const uint32_t nch = ex ? (nd.count + B_PART_CHUNK - 1) / B_PART_CHUNK : 0u;
-        const uint32_t jc = block_excl_scan(nch, sh, &tc);
+        uint32_t te, tc, je, jc;  // expansions and their row chunks in one scan
+        block_excl_scan2(ex ? 1u : 0u, nch, sh, &je, &jc, &te, &tc);
+        const uint32_t n_tile = min(nf - i0, blockDim.x), tl = n_tile - te, jl = threadIdx.x - je;
         if (valid && !ex) {
             const float v = leaf_value_dev(nd.G, nd.H, scale, lp);
             write_leaf(d.tree[nd.tnode], nd.G, nd.H, scale, v);
@@ -2938,86 +3192,111 @@ __device__ void write_chunk_owners(uint2* map, uint32_t cap, uint32_t base, uint
     }
 }
 
+// Rows per histogram row segment for `rows` rows: about hist_target segments
+// (a multiple of 256 rows in [1024, hist_seg_max]), so that the persistent
+// histogram launch has a few equal items per block; node sums (last level) use
+// HIST_CHUNK_MAX-row chunks.
+__device__ __forceinline__ uint32_t level_chunk(const BDev& d, unsigned long long rows, int need_split) {
+    if (!need_split) return HIST_CHUNK_MAX;
+    const uint32_t tgt = d.hist_target ? d.hist_target : 1u;
+    unsigned long long want = (rows + tgt - 1) / tgt;
+    want = (want + 255ull) & ~255ull;
+    return (uint32_t)(want < 1024ull ? 1024ull : (want > d.hist_seg_max ? d.hist_seg_max : want));
+}
+
 __device__ void children_body(BDev d, int a, int need_split) {
-    __shared__ uint32_t sh[33];
+    __shared__ uint32_t sh[66];
     __shared__ uint32_t s_jc[PART_THREADS], s_own[PART_THREADS];  // block size of its caller, k_b_partition
-    __shared__ uint32_t base, n_exp, chunk;
-    __shared__ unsigned long long rows;
+    __shared__ uint32_t base, s_exp;
     BState* s = d.state;
     if (threadIdx.x == 0) {
-        n_exp = s->n_exp;
+        s_exp = s->n_exp;
         base = 0;
-        rows = 0ull;
     }
     __syncthreads();
+    const uint32_t n_exp = s_exp;
     const BNode* A = d.front[a];
     BNode* B = d.front[a ^ 1];
-    for (uint32_t j0 = 0; j0 < n_exp; j0 += blockDim.x) {
-        const uint32_t j = j0 + threadIdx.x;
+    // the children of expansion j (all but its hist_off)
+    auto child = [&](uint32_t j) {
+        BExp e = d.exp[j];
+        const uint4 nd = *reinterpret_cast<const uint4*>(&A[e.front]);  // pnode, tnode, begin, count
+        const uint32_t lc = d.cursors[2 * j] - nd.z, rc = nd.w - lc;
+        const bool left_small = lc <= rc;
+        e.lc = lc;
+        e.rc = rc;
+        e.small_begin = left_small ? nd.z : nd.z + lc;
+        e.small_count = left_small ? lc : rc;
+        BNode l, r;
+        l.pnode = nd.x;
+        l.tnode = e.tl;
+        l.begin = nd.z;
+        l.count = lc;
+        r.pnode = e.right_pnode;
+        r.tnode = e.tr;
+        r.begin = nd.z + lc;
+        r.count = rc;
+        l.G = l.H = r.G = r.H = 0;
+        l.split.gain = r.split.gain = -INFINITY;
+        l.split.col = r.split.col = 0;
+        l.split.bin = r.split.bin = 0;
+        l.split.flags = r.split.flags = 0;
+        for (int q = 0; q < 4; ++q) l.split.cats[q] = r.split.cats[q] = 0ull;
+        l.split.tot_g = l.split.tot_h = r.split.tot_g = r.split.tot_h = 0;
+        B[2 * j] = l;
+        B[2 * j + 1] = r;
+        // row sampling: the split search counts the sampled rows
+        const uint32_t slc = d.rmask ? d.scnt[2 * j] : lc, src = d.rmask ? d.scnt[2 * j + 1] : rc;
+        d.scan_nodes[2 * j] = ScanNode{nd.x, slc, 0u, 0u, 0, 0};
+        d.scan_nodes[2 * j + 1] = ScanNode{e.right_pnode, src, 0u, 0u, 0, 0};
+        return e;
+    };
+    unsigned long long rows = 0;
+    uint32_t chunk;
+    if (n_exp <= blockDim.x) {  // a thread per expansion, kept in registers
+        const uint32_t j = threadIdx.x;
         const bool valid = j < n_exp;
+        BExp e;
+        e.small_count = 0;
+        if (valid) e = child(j);
+        uint32_t x0, x1, t0, t1;
+        block_excl_scan2(e.small_count, 0u, sh, &x0, &x1, &t0, &t1);  // rows fit 32 bits
+        rows = t0;
+        chunk = level_chunk(d, rows, need_split);
+        const uint32_t nch = (e.small_count + chunk - 1) / chunk;
+        block_excl_scan2(nch, 0u, sh, &x0, &x1, &t0, &t1);
         if (valid) {
-            BExp e = d.exp[j];
-            const BNode nd = A[e.front];
-            const uint32_t lc = d.cursors[2 * j] - nd.begin, rc = nd.count - lc;
-            const bool left_small = lc <= rc;
-            e.lc = lc;
-            e.rc = rc;
-            e.small_begin = left_small ? nd.begin : nd.begin + lc;
-            e.small_count = left_small ? lc : rc;
-            BNode l, r;
-            l.pnode = nd.pnode;
-            l.tnode = e.tl;
-            l.begin = nd.begin;
-            l.count = lc;
-            r.pnode = e.right_pnode;
-            r.tnode = e.tr;
-            r.begin = nd.begin + lc;
-            r.count = rc;
-            l.G = l.H = r.G = r.H = 0;
-            l.split.gain = r.split.gain = -INFINITY;
-            l.split.col = r.split.col = 0;
-            l.split.bin = r.split.bin = 0;
-            l.split.flags = r.split.flags = 0;
-            for (int q = 0; q < 4; ++q) l.split.cats[q] = r.split.cats[q] = 0ull;
-            l.split.tot_g = l.split.tot_h = r.split.tot_g = r.split.tot_h = 0;
-            B[2 * j] = l;
-            B[2 * j + 1] = r;
-            // row sampling: the split search counts the sampled rows
-            const uint32_t slc = d.rmask ? d.scnt[2 * j] : lc, src = d.rmask ? d.scnt[2 * j + 1] : rc;
-            d.scan_nodes[2 * j] = ScanNode{nd.pnode, slc, 0u, 0u, 0, 0};
-            d.scan_nodes[2 * j + 1] = ScanNode{e.right_pnode, src, 0u, 0u, 0, 0};
+            e.hist_off = x0;
             d.exp[j] = e;
-            atomicAdd(&rows, (unsigned long long)e.small_count);
         }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        // rows per histogram row segment: about hist_target segments (a
-        // multiple of 256 rows in [1024, hist_seg_max]), so that the
-        // persistent histogram launch has a few equal items per block; node
-        // sums (last level) use HIST_CHUNK_MAX-row chunks
-        uint32_t c = HIST_CHUNK_MAX;
-        if (need_split) {
-            const uint32_t tgt = d.hist_target ? d.hist_target : 1u;
-            unsigned long long want = (rows + tgt - 1) / tgt;
-            want = (want + 255ull) & ~255ull;
-            c = (uint32_t)(want < 1024ull ? 1024ull : (want > d.hist_seg_max ? d.hist_seg_max : want));
+        write_segment_owners(d.seg_exp, d.max_segs, 0u, x0, j, t0, s_jc, s_own);  // segment -> expansion
+        if (j == 0) base = t0;
+        __syncthreads();
+    } else {
+        __shared__ unsigned long long s_rows;
+        if (threadIdx.x == 0) s_rows = 0ull;
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < n_exp; j += blockDim.x) {
+            const BExp e = child(j);
+            d.exp[j] = e;
+            atomicAdd(&s_rows, (unsigned long long)e.small_count);
         }
-        chunk = c;
-    }
-    __syncthreads();
-    for (uint32_t j0 = 0; j0 < n_exp; j0 += blockDim.x) {
-        const uint32_t j = j0 + threadIdx.x;
-        const bool valid = j < n_exp;
-        const uint32_t nch = valid ? (d.exp[j].small_count + chunk - 1) / chunk : 0u;
-        uint32_t tc;
-        const uint32_t jc = block_excl_scan(nch, sh, &tc);
-        if (valid) d.exp[j].hist_off = base + jc;
-        // segment -> expansion (the buffer bound always holds)
-        write_segment_owners(d.seg_exp, d.max_segs, base, jc, j, tc, s_jc, s_own);
         __syncthreads();
-        if (threadIdx.x == 0) base += tc;
-        __syncthreads();
+        rows = s_rows;
+        chunk = level_chunk(d, rows, need_split);
+        for (uint32_t j0 = 0; j0 < n_exp; j0 += blockDim.x) {
+            const uint32_t j = j0 + threadIdx.x;
+            const bool valid = j < n_exp;
+            const uint32_t nch = valid ? (d.exp[j].small_count + chunk - 1) / chunk : 0u;
+            uint32_t jc, z, tc, tz;
+            block_excl_scan2(nch, 0u, sh, &jc, &z, &tc, &tz);
+            if (valid) d.exp[j].hist_off = base + jc;
+            // segment -> expansion (the buffer bound always holds)
+            write_segment_owners(d.seg_exp, d.max_segs, base, jc, j, tc, s_jc, s_own);
+            __syncthreads();
+            if (threadIdx.x == 0) base += tc;
+            __syncthreads();
+        }
     }
     if (!need_split)  // the node sums of k_b_sums accumulate from zero
         for (uint32_t i = threadIdx.x; i < 2 * n_exp; i += blockDim.x) d.sums[i] = 0;
@@ -3763,36 +4042,39 @@ __device__ __forceinline__ unsigned long long cand_key(float g, uint32_t col, in
 // frontier b's splits (the winner's full candidate from cand), resets the
 // keys, and derives the next level's decisions (rows in buffer buf).
 template <typename HB>
-__global__ void __launch_bounds__(SCAN_WARPS * 32, 4)
+__global__ void __launch_bounds__(SCAN_WARPS * 32, 3)
 k_b_scan(BDev d, const ScanColumn* __restrict__ cols, uint32_t n_cols, const HB* __restrict__ hist,
          uint64_t slot_bins, const double* __restrict__ scale, GainParamsDev gp, ColCand* __restrict__ cand,
          long long* __restrict__ node_tot, int b, int last_wins, LeafParams lp, uint32_t buf,
          const ScanNode* __restrict__ root, const uint8_t* __restrict__ colmask, NodeSplit* __restrict__ lw_out) {
     BST_PDL_ENTER();
-    __shared__ double s_key[SCAN_WARPS][SORT_N];
-    __shared__ uint32_t s_cat[SCAN_WARPS][SORT_N];
+    __shared__ __align__(16) unsigned char scratch[SCAN_WARPS][scan_scratch<HB>()];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n_nodes = root ? 1u : 2 * d.state->n_exp;
     const uint32_t col_blocks = (n_cols + SCAN_WARPS - 1) / SCAN_WARPS;
     const uint64_t items = (uint64_t)n_nodes * col_blocks;
-    for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
-        const uint32_t node = (uint32_t)(it / col_blocks);
-        const uint32_t col = (uint32_t)(it % col_blocks) * SCAN_WARPS + warp;
-        if (col < n_cols) {
-            const ScanNode nd = root ? root[0] : d.scan_nodes[node];
-            const float g = scan_item(nd, node, col, cols, n_cols, hist, slot_bins, scale, gp, cand, node_tot,
-                                      s_key[warp], s_cat[warp], colmask ? colmask + (size_t)nd.pad * n_cols : nullptr);
-            if (lane == 0 && g > -INFINITY) atomicMax(&d.node_key[node], cand_key(g, col, last_wins));
+    if (blockIdx.x < items) {
+        const ScanUnits un(scale, gp);
+        for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
+            const uint32_t node = (uint32_t)(it / col_blocks);
+            const uint32_t col = (uint32_t)(it % col_blocks) * SCAN_WARPS + warp;
+            if (col < n_cols) {
+                const ScanNode nd = root ? root[0] : d.scan_nodes[node];
+                const float g = scan_item(nd, cols[col], node, col, n_cols, hist, slot_bins, scale, un, gp, cand, node_tot,
+                                          scratch[warp], colmask ? colmask + (size_t)nd.pad * n_cols : nullptr);
+                if (lane == 0 && g > -INFINITY) atomicMax(&d.node_key[node], cand_key(g, col, last_wins));
+            }
         }
     }
     if (!last_block(d.state)) return;
     BNode* B = d.front[b];
-    for (uint32_t node = threadIdx.x; node < n_nodes; node += blockDim.x) {
+    // the winner of one node: its split, the key reset
+    auto winner = [&](uint32_t node) {
         const unsigned long long key = d.node_key[node];
-        d.node_key[node] = 0ull;
         NodeSplit sp;
         sp.tot_g = node_tot[2 * node];
         sp.tot_h = node_tot[2 * node + 1];
+        d.node_key[node] = 0ull;
         if (key == 0ull) {
             sp.gain = -INFINITY;
             sp.col = 0;
@@ -3808,15 +4090,18 @@ k_b_scan(BDev d, const ScanColumn* __restrict__ cols, uint32_t n_cols, const HB*
             sp.flags = (w.flags & 3u) | 4u;
             for (int q = 0; q < 4; ++q) sp.cats[q] = w.cats[q];
         }
-        if (lw_out) {
-            lw_out[node] = sp;
-            continue;
-        }
+        return sp;
+    };
+    if (lw_out) {
+        for (uint32_t node = threadIdx.x; node < n_nodes; node += blockDim.x) lw_out[node] = winner(node);
+        return;
+    }
+    for (uint32_t node = threadIdx.x; node < n_nodes; node += blockDim.x) {
+        const NodeSplit sp = winner(node);
         B[node].split = sp;
         B[node].G = sp.tot_g;
         B[node].H = sp.tot_h;
     }
-    if (lw_out) return;
     __syncthreads();
     decide_body(d, b, lp, scale, buf);
 }

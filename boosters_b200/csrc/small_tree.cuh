@@ -142,46 +142,6 @@ __device__ __forceinline__ unsigned long long st_candidates(T2 P, T2 T, T2 M, ui
     return best;
 }
 
-// Sums of hessians from hmin on pass `(double)h * ih >= mcw`, none below do
-// (the product is monotone in h); exact: hmin is known (else the test itself
-// is made).
-struct StMin {
-    long long h;
-    bool exact;
-};
-__device__ __forceinline__ StMin st_min(double mcw, double ih) {
-    StMin r{0, false};
-    const double h0 = mcw / ih;
-    if (!(fabs(h0) < 1.0e15)) return r;
-    r.h = (long long)floor(h0) - 2;
-    for (int i = 0; i < 6; ++i)
-        if (!((double)r.h * ih >= mcw)) ++r.h;
-    r.exact = (double)r.h * ih >= mcw && !((double)(r.h - 1) * ih >= mcw);
-    return r;
-}
-
-// Largest approximate score of one lane's valid candidates (those of
-// st_candidates): -1 when there is none, infinity when it cannot be bounded.
-template <typename T2>
-__device__ __forceinline__ float st_scores(T2 P, T2 T, T2 M, uint32_t b, uint32_t nb, bool hm, uint32_t pc,
-                                           const StMin& hmin, float lam, double mcw, double ih, uint32_t msl) {
-    float best = -1.0f;
-    auto one = [&](long long lg, long long lh, long long rg, long long rh, uint32_t lc, uint32_t rc) {
-        const bool w = hmin.exact ? (lh >= hmin.h && rh >= hmin.h) : ((double)lh * ih >= mcw && (double)rh * ih >= mcw);
-        if (!w || lc < msl || rc < msl) return;
-        const float dl = (float)lh + lam, dr = (float)rh + lam;
-        const float gl = (float)lg, gr = (float)rg;
-        const float sc = __fdividef(gl * gl, dl) + __fdividef(gr * gr, dr);
-        best = lh >= 0 && rh >= 0 && dl > 0.0f && dr > 0.0f && sc < INFINITY ? fmaxf(best, sc) : INFINITY;
-    };
-    if (b + 1 < nb) one(P.x, P.y, (long long)T.x - P.x, (long long)T.y - P.y, b + 1, sat_sub(pc, b + 1));
-    if (hm && b + 2 < nb) {
-        const long long Rg = (long long)M.x - P.x, Rh = (long long)M.y - P.y;
-        one((long long)T.x - Rg, (long long)T.y - Rh, Rg, Rh, sat_sub(pc, nb - 2 - b), nb - 2 - b);
-    }
-    return best;
-}
-
 struct StShared {  // the level's facts, the same in every block
     PartWork work[ST_FRONT / 2];     // expansions: split rule (begin / count unused)
     uint16_t tl[ST_FRONT / 2], tr[ST_FRONT / 2];  // tree nodes of the training-left / right child
@@ -196,7 +156,7 @@ struct StShared {  // the level's facts, the same in every block
     uint32_t sh[33];
     uint32_t first_col, n_list;
     longlong2 ptot[ST_FRONT / 2];    // the expansions' totals
-    StMin hmin;
+    HessMin hmin;
     float lam;                       // lambda in units of the hessian sums
     ScanColumn col;   // of column blockIdx.x
     BColumn bcol;
@@ -478,9 +438,10 @@ __device__ void st_histograms(const SmallTree& a, StShared& s, unsigned char* dy
                         const uint32_t side = (kid == 0u) == sl ? 0u : 1u;
                         const longlong2 T = kid ? make_longlong2(Tp.x - Ts.x, Tp.y - Ts.y) : Ts;
                         const longlong2 M = kid ? make_longlong2(mp.x - ms.x, mp.y - ms.y) : ms;
-                        float sc = st_scores(kid ? pl : ps, T, M, b, B, hm, s.f_cnt[root ? 0u : 2u * (j0 + j) + side],
-                                             s.hmin, s.lam, a.gp.min_child_weight, ih, a.gp.min_samples_leaf);
-                        if (!(a.gp.min_gain >= 0.0) || T.y < 0 || !((float)T.y + s.lam > 0.0f))
+                        const ScoreRule<long long> rule(s.hmin, s.lam, a.gp, ih,
+                                                        s.f_cnt[root ? 0u : 2u * (j0 + j) + side]);
+                        float sc = rule.best(kid ? pl : ps, T, M, b, B, hm);
+                        if (sc >= 0.0f && (!(a.gp.min_gain >= 0.0) || T.y < 0 || !((float)T.y + s.lam > 0.0f)))
                             sc = INFINITY;  // the offset's sign is not known
                         for (int o = 16; o > 0; o >>= 1) sc = fmaxf(sc, __shfl_xor_sync(FULL, sc, o));
                         if (lane == 0u) score[2u * (j * nq + q) + side] = sc;
@@ -588,9 +549,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_small_tree(const __grid_const
     if (tid < 4u) s.scale[tid] = a.scale[tid];
     if (tid == 64u) {
         s.first_col = 0u;
-        s.hmin = st_min(a.gp.min_child_weight, a.scale[3]);
-        const double lam = a.gp.lambda / a.scale[3];
-        s.lam = lam >= 0.0 && lam < 1.0e36 ? (float)lam : -INFINITY;  // out of range: no filter
+        s.hmin = hess_min(a.gp.min_child_weight, a.scale[3]);
+        s.lam = hess_lambda(a.gp.lambda, a.scale[3]);
     }
     if (tid == 32u && blockIdx.x < a.n_cols) {
         s.col = a.cols[blockIdx.x];
