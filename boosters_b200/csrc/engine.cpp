@@ -1658,7 +1658,7 @@ class Trainer {
         return host_tree_from(std::move(t), st->n_tnodes, reinterpret_cast<const BTreeNode*>(sl.small + sizeof(BState)));
     }
 
-    // ---- device-side level loop, one CUDA graph per output (kernels.h) -------
+    // ---- device-side level loop (kernels.h); with cuda_graph, a graph per output
     bool use_batched_ = false;
     // batched leaf-wise: speculative expansion batches, gradient elements
     // carried positionally in qpos_[0] (aligned with ridx_), split columns
@@ -2051,6 +2051,27 @@ class Trainer {
         launches += 2;
     }
 
+    // What f enqueues on the stream, as an executable graph.
+    template <class F>
+    cudaGraphExec_t capture(F f) {
+        BST_CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
+        try {
+            f();
+        } catch (...) {
+            cudaGraph_t g = nullptr;
+            cudaStreamEndCapture(st_, &g);
+            if (g) cudaGraphDestroy(g);
+            throw;
+        }
+        cudaGraph_t g = nullptr;
+        BST_CK(cudaStreamEndCapture(st_, &g));
+        cudaGraphExec_t ex = nullptr;
+        const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+        cudaGraphDestroy(g);
+        BST_CK(e);
+        return ex;
+    }
+
     // Enqueues the tree of output o into ring slot `si` (no host wait).
     void launch_batched(uint32_t o, uint32_t si) {
         if (use_small_) return launch_small(o, si);
@@ -2065,37 +2086,41 @@ class Trainer {
             sl.cand = c;
             sl.timed = timed;
         }
-        if (!graphs_[gi]) {
+        if (!gtimers_[gi]) {
             gtimers_[gi] = std::make_unique<Timer>();
             gtimers_[gi]->st = st_;
             gtimers_[gi]->enabled = cfg_.phase_timings != 0;
             gtimers_[gi]->reserve(16 + 20 * (size_t)cfg_.max_depth);
-            gtimers_[gi]->in_graph = true;
-            bd_.rmask = rowmask(o);  // baked into the graph's kernels
-            BST_CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
-            try {
-                enqueue_tree(o, *gtimers_[gi], graph_launches_[gi], graph_hist_launches_[gi]);
-            } catch (...) {
-                cudaGraph_t g = nullptr;
-                cudaStreamEndCapture(st_, &g);
-                if (g) cudaGraphDestroy(g);
-                throw;
-            }
-            cudaGraph_t g = nullptr;
-            BST_CK(cudaStreamEndCapture(st_, &g));
-            cudaGraphExec_t ex = nullptr;
-            const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
-            cudaGraphDestroy(g);
-            BST_CK(e);
-            graphs_[gi] = ex;
+            gtimers_[gi]->in_graph = cfg_.cuda_graph != 0;
         }
-        upload_col_masks(o, si);  // read by the graph's split searches
+        Timer& gt = *gtimers_[gi];
+        bd_.rmask = rowmask(o);
+        if (cfg_.cuda_graph && !graphs_[gi]) {
+            gt.marks.clear();
+            gt.used = 0;
+            graphs_[gi] = capture([&] { enqueue_tree(o, gt, graph_launches_[gi], graph_hist_launches_[gi]); });
+        }
+        upload_col_masks(o, si);  // read by the tree's split searches
         if (rowsample_) {  // the root's split search counts the sampled rows
             const ScanNode rs{0, n_sampled_[o], 0u, 0u, 0, 0};
             BST_CK(cudaMemcpyAsync(d_root_scan_.p, &rs, sizeof(rs), cudaMemcpyHostToDevice, st_));
         }
         BST_CK(cudaEventRecord(sl.w0, st_));
-        BST_CK(cudaGraphLaunch(graphs_[gi], st_));
+        // Launched one by one unless the caller asked for graphs: even a tree
+        // of 100K rows takes 280 us, several times what its launches take, and
+        // the ring lets the host run ahead, so a graph's replay gains nothing
+        // (281 and 283 us there, 696 and 698 us a q8 tree of 1M x 100), while
+        // capturing and instantiating one, 0.35 ms, came again with every launch
+        // shape explored and for every output (43.5 against 39.4 ms a call of
+        // 50 early-stopped trees).
+        if (cfg_.cuda_graph) {
+            BST_CK(cudaGraphLaunch(graphs_[gi], st_));
+        } else {
+            gt.marks.clear();
+            gt.used = 0;
+            enqueue_tree(o, gt, graph_launches_[gi], graph_hist_launches_[gi]);
+            BST_CK(cudaGetLastError());
+        }
         BST_CK(cudaEventRecord(sl.w1, st_));
         BST_CK(cudaMemcpyAsync(sl.state, d_bstate_.p, sizeof(BState), cudaMemcpyDeviceToHost, st_));
         BST_CK(cudaMemcpyAsync(sl.tree, d_btree_.p, sizeof(BTreeNode) * max_tnodes_, cudaMemcpyDeviceToHost, st_));
@@ -2692,7 +2717,7 @@ class Trainer {
 
     // ---- batched leaf-wise growth on the device (kernels.h, k_lw_replay) -----
     // The replay of the heap pops runs on the device between expansion
-    // steps; the host launches LW_STEPS steps at a time as one CUDA graph and
+    // steps; the host launches LW_STEPS steps at a time (cuda_graph: as a graph) and
     // reads back only whether the tree is done.
     static constexpr uint32_t LW_STEPS = 6;
     DevArray<LwState> d_lw_state_;
@@ -2761,7 +2786,7 @@ class Trainer {
             t = std::make_unique<Timer>();
             t->st = st_;
             t->enabled = cfg_.phase_timings != 0;
-            t->in_graph = true;
+            t->in_graph = cfg_.cuda_graph != 0;
             t->reserve(LW_STEPS * 12 + 4);
         }
     }
@@ -2840,31 +2865,23 @@ class Trainer {
         timer_.end();
         launch_lw_init(bd_, lw_, (uint32_t)n_, (uint32_t)n_, st_);
         m_.counters.launches += 5;
-        // expansion steps, LW_STEPS per graph launch, until the replay is done
-        if (!lw_graphs_[o]) {
-            BST_CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
-            try {
-                enqueue_lw_steps(o, *lw_timers_[o], lw_launches_[o], lw_hist_launches_[o]);
-            } catch (...) {
-                cudaGraph_t g = nullptr;
-                cudaStreamEndCapture(st_, &g);
-                if (g) cudaGraphDestroy(g);
-                throw;
-            }
-            cudaGraph_t g = nullptr;
-            BST_CK(cudaStreamEndCapture(st_, &g));
-            cudaGraphExec_t ex = nullptr;
-            const cudaError_t ce = cudaGraphInstantiate(&ex, g, 0);
-            cudaGraphDestroy(g);
-            BST_CK(ce);
-            lw_graphs_[o] = ex;
-        }
+        // expansion steps, LW_STEPS at a time, until the replay is done
+        if (cfg_.cuda_graph && !lw_graphs_[o])
+            lw_graphs_[o] =
+                capture([&] { enqueue_lw_steps(o, *lw_timers_[o], lw_launches_[o], lw_hist_launches_[o]); });
         // each step but the last pops at least one leaf
         const uint32_t max_launches = cfg_.max_leaves / LW_STEPS + 4;
         Timer& gt = *lw_timers_[o];
         for (uint32_t it = 0;; ++it) {
             if (it > max_launches) throw Error{BST_ERR_CUDA, "leaf-wise replay did not finish"};
-            BST_CK(cudaGraphLaunch(lw_graphs_[o], st_));
+            if (cfg_.cuda_graph) {
+                BST_CK(cudaGraphLaunch(lw_graphs_[o], st_));
+            } else {  // (as launch_batched: a step's kernels outlast their launches)
+                gt.marks.clear();
+                gt.used = 0;
+                enqueue_lw_steps(o, gt, lw_launches_[o], lw_hist_launches_[o]);
+                BST_CK(cudaGetLastError());
+            }
             BST_CK(cudaMemcpyAsync(h_lw_state_, d_lw_state_.p, sizeof(LwState), cudaMemcpyDeviceToHost, st_));
             BST_CK(cudaStreamSynchronize(st_));
             if (gt.enabled && gt.collect_keep())

@@ -295,10 +295,10 @@ struct LeafSeg {
 void launch_leaf_update(const LeafSeg* leaves, uint32_t n_leaves, const uint32_t* ridx,
                         uint64_t n, float* pred, uint32_t* row_leaf, cudaStream_t st);
 
-// ---- device-side depth-wise growth (one CUDA graph per tree) -----------------
+// ---- device-side depth-wise growth --------------------------------------------
 // The host launches a fixed sequence of kernels per tree; every data-dependent
 // size (frontier, expanding nodes, row chunks) is read from device memory, so
-// the sequence is captured once and replayed for every tree.
+// the sequence is the same for every tree (and can be captured once).
 struct BColumn {  // per effective column, for decisions and the partition
     uint32_t matrix, pos, has_missing, default_bin;
 };
