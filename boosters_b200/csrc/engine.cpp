@@ -1680,6 +1680,7 @@ class Trainer {
     DevArray<uint32_t> d_bin_map_;  // global bin -> (lane tile, partial entry)
     DevArray<uint2> d_ent_;         // node partial entry -> (global bin, lane tile / offset)
     uint32_t n_ent_ = 0;
+    DevArray<uint32_t> d_col_part_; // column -> (lane tile, its first partial entry), or none
     DevArray<ScanNode> d_root_scan_;
     uint32_t max_tnodes_ = 0;
     // Pipelined replay: tree k is read back and converted on the host while
@@ -1754,6 +1755,7 @@ class Trainer {
         d_seg_exp_.alloc(max_segs);
         bd_.seg_exp = d_seg_exp_.p;
         bd_.max_segs = (uint32_t)max_segs;
+        std::vector<uint32_t> cp(std::max<uint32_t>(1, n_cols_), 0xFFFFFFFFu);
         if (n_lane_tiles_) {
             d_part_.alloc(max_segs * n_lane_tiles_ * (size_t)lane_part_stride() * lane_part_entry_bytes(qmode_));
             std::vector<uint32_t> bm(p_.total_bins, 0xFFFFFFFFu);
@@ -1771,12 +1773,16 @@ class Trainer {
             n_ent_ = (uint32_t)ent.size();
             d_ent_.alloc(std::max<size_t>(1, ent.size()));
             BST_CK(cudaMemcpy(d_ent_.p, ent.data(), sizeof(uint2) * ent.size(), cudaMemcpyHostToDevice));
+            for (uint32_t c = 0; c < n_cols_; ++c)
+                if (p_.col_nbins[c]) cp[c] = bm[p_.col_hist_off[c]];
             d_bin_map_.alloc(p_.total_bins);
             BST_CK(cudaMemcpy(d_bin_map_.p, bm.data(), sizeof(uint32_t) * bm.size(), cudaMemcpyHostToDevice));
         } else {
             d_bin_map_.alloc(std::max<uint64_t>(1, p_.total_bins));
             BST_CK(cudaMemset(d_bin_map_.p, 0xFF, sizeof(uint32_t) * std::max<uint64_t>(1, p_.total_bins)));
         }
+        d_col_part_.alloc(cp.size());
+        BST_CK(cudaMemcpy(d_col_part_.p, cp.data(), sizeof(uint32_t) * cp.size(), cudaMemcpyHostToDevice));
     }
 
     // ---- launch-shape autotuning (autotune.h) ----------------------------------
@@ -1936,12 +1942,19 @@ class Trainer {
     // Histograms of the smaller children described by the level state in bd_
     // (or of all rows, root): partial histograms of the lane tiles, general
     // tiles (atomic, into zeroed right slots), then the merge with the
-    // subtraction trick.
-    // wide: the level has at most WIDE_MERGE_NODES expanding nodes (the
-    // merge splits each node's many row segments over more threads)
+    // subtraction trick: of the general tiles alone where the level's split
+    // search (launch_b_scan) merges the lane tiles, of all for the searches that
+    // read merged histograms, there wide if the level has at most
+    // WIDE_MERGE_NODES expanding nodes (the merge splits each node's many row
+    // segments over more threads).
     static constexpr uint32_t WIDE_MERGE_NODES = 4;
+    // A root of more segments than this is merged apart: its search has one
+    // block a column, too few to read them (fp32, 245 segments of 100 columns:
+    // merge and search 35 us apart, 41 in one; q8, 62 segments: 18.2 and 18.8).
+    static constexpr uint32_t ROOT_SCAN_SEGS = 128;
+    enum class Merge { General, All, AllWide };
     void enqueue_hist(const GradRef& gr, const uint32_t* ridx, bool root, Timer& tm, uint64_t& launches,
-                      uint64_t& hist_launches, bool wide = false) {
+                      uint64_t& hist_launches, Merge merge) {
         // resident general-tile blocks per SM: 64 registers x 256 threads
         // allow 4; the fixed-point form's 16 B/bin shared histograms allow 3
         const uint32_t g_hist = sm_count() * (qmode_ == GRAD_F32 ? 3 : 4);
@@ -1953,12 +1966,15 @@ class Trainer {
             launch_b_hist(bd_, tiles_.p, n_tiles_, tile_smem_, ridx, gr, b_.bins8, p_.s8, b_.bins16, p_.s16,
                           hist_.p, slot_bins_, g_hist, st_, hist32_);
         tm.end();
-        tm.begin(PH_OTHER);
-        launch_b_merge(bd_, hist_.p, slot_bins_, p_.total_bins, d_part_.p, n_lane_tiles_, d_ent_.p, n_ent_,
-                       d_bin_map_.p, n_tiles_ > 0, root ? 1 : 0, qmode_, st_, hist32_, wide ? 1 : 0);
-        tm.end();
         const uint32_t hist_kernels = (n_lane_tiles_ ? 1u : 0u) + (n_tiles_ ? 1u : 0u);
-        launches += 2 * hist_kernels;  // builds and merges
+        const uint32_t merged = merge == Merge::General ? 0u : n_lane_tiles_;
+        if (merged || n_tiles_) {
+            tm.begin(PH_OTHER);
+            launch_b_merge(bd_, hist_.p, slot_bins_, p_.total_bins, d_part_.p, merged, d_ent_.p, n_ent_, d_bin_map_.p,
+                           n_tiles_ > 0, root ? 1 : 0, qmode_, st_, hist32_, merge == Merge::AllWide ? 1 : 0);
+            tm.end();
+        }
+        launches += hist_kernels + (merged ? 1u : 0u) + (n_tiles_ ? 1u : 0u);  // builds and merges
         hist_launches += hist_kernels;
     }
 
@@ -1975,17 +1991,17 @@ class Trainer {
         // items (idle blocks would still take part in the last-block
         // hand-off): split searches 2^(d+1) nodes x column blocks,
         // partitions n / chunk + 2^d chunks, leaf kernels n / chunk + leaves
-        const uint64_t cb = scan_col_blocks(n_cols_);
         auto cap = [&](uint64_t items) { return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(g_wide, items)); };
         tm.begin(PH_OTHER);
         launch_b_root_init(bd_, ridx_.p, n_, chunk_rows(n_), st_);  // row ids, root node, root histogram state
         if (n_tiles_) BST_CK(cudaMemsetAsync(hist_.p, 0, hbytes() * slot_bins_, st_));
         tm.end();
-        enqueue_hist(gh, ridx_.p, true, tm, launches, hist_launches, true);
+        const bool root_merge = (n_ + chunk_rows(n_) - 1) / chunk_rows(n_) > ROOT_SCAN_SEGS;
+        enqueue_hist(gh, ridx_.p, true, tm, launches, hist_launches, root_merge ? Merge::AllWide : Merge::General);
         tm.begin(PH_SCAN);
-        launch_b_scan(bd_, scan_cols_.p, n_cols_, hist_.p, slot_bins_, scale, gp_, d_cand_.p, d_node_tot_.p, 0,
-                      last_wins_ ? 1 : 0, lp, 0u, cap(cb), st_, hist32_, d_root_scan_.p,
-                      colmask());  // + level-0 decisions
+        launch_b_scan(bd_, scan_cols_.p, n_cols_, root_merge ? nullptr : d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p, slot_bins_,
+                      cfg_.max_depth > 1, scale, gp_, d_cand_.p, d_node_tot_.p, 0, last_wins_ ? 1 : 0, lp, 0u, 1u, g_wide,
+                      st_, hist32_, d_root_scan_.p, colmask());  // + level-0 decisions
         tm.end();
         launches += 2;  // root init, root split search
         // row indices: level d partitions R[d & 1] into R[(d + 1) & 1]
@@ -2012,12 +2028,14 @@ class Trainer {
                     tm.end();
                     launches += 1;
                 }
-                // level d expands at most 2^d nodes
-                enqueue_hist(gl, rout, false, tm, launches, hist_launches, (1u << std::min(d, 31u)) <= WIDE_MERGE_NODES);
+                enqueue_hist(gl, rout, false, tm, launches, hist_launches, Merge::General);
                 tm.begin(PH_SCAN);
-                launch_b_scan(bd_, scan_cols_.p, n_cols_, hist_.p, slot_bins_, scale, gp_, d_cand_.p,
-                              d_node_tot_.p, a ^ 1, last_wins_ ? 1 : 0, lp, (d + 1) & 1u, cap((2ull << d) * cb), st_, hist32_,
-                              nullptr, colsample_ ? d_colmask_.p + (size_t)(d + 1) * n_cols_ : nullptr);
+                // level d expands at most 2^d nodes; its children's histograms
+                // are read again unless their children are leaves
+                launch_b_scan(bd_, scan_cols_.p, n_cols_, d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p,
+                              slot_bins_, d + 2 < cfg_.max_depth, scale, gp_, d_cand_.p, d_node_tot_.p, a ^ 1,
+                              last_wins_ ? 1 : 0, lp, (d + 1) & 1u, 1u << std::min(d, 31u), g_wide, st_, hist32_, nullptr,
+                              colsample_ ? d_colmask_.p + (size_t)(d + 1) * n_cols_ : nullptr);
                 // + column reduction, next level's decisions
                 tm.end();
                 launches += 1;
@@ -2270,7 +2288,8 @@ class Trainer {
         upload(hs, 1, d_bstate_);
         upload(hseg, segs.size(), d_seg_exp_);
         uint64_t launches = 0, hist_launches = 0;
-        enqueue_hist(gr_o_, ridx_.p, root, timer_, launches, hist_launches, exps.size() <= WIDE_MERGE_NODES);
+        enqueue_hist(gr_o_, ridx_.p, root, timer_, launches, hist_launches,
+                     exps.size() <= WIDE_MERGE_NODES ? Merge::AllWide : Merge::All);
         m_.counters.launches += launches;
         m_.counters.hist_launches += hist_launches;
         m_.counters.hist_rows += rows;
@@ -2562,7 +2581,8 @@ class Trainer {
         launch_lw_children(bd_, d_pworks_.p, d_cursors_.p, (uint32_t)k, d_scan_nodes_.p,
                            rowsample_ ? d_scnt_.p : nullptr, st_);
         uint64_t launches = 1, hist_launches = 0;
-        enqueue_hist(gr_o_, ridx_.p, false, timer_, launches, hist_launches, k <= WIDE_MERGE_NODES);
+        enqueue_hist(gr_o_, ridx_.p, false, timer_, launches, hist_launches,
+                     k <= WIDE_MERGE_NODES ? Merge::AllWide : Merge::All);
         timer_.begin(PH_SCAN);
         launch_split_scan(d_scan_nodes_.p, (uint32_t)(2 * k), scan_cols_.p, n_cols_, hist_.p, slot_bins_, scale_o_, gp_,
                           d_cand_.p, d_node_tot_.p, st_, hist32_, colmask());
@@ -2824,10 +2844,11 @@ class Trainer {
                                rowsample_ ? d_scnt_.p : nullptr, st_);
             if (n_tiles_) launch_b_zero_right(bd_, hist_.p, slot_bins_, g_wide_, st_, hist32_);
             tm.end();
-            enqueue_hist(gr, ridx_.p, false, tm, launches, hist_launches, false);
+            enqueue_hist(gr, ridx_.p, false, tm, launches, hist_launches, Merge::General);
             tm.begin(PH_SCAN);
-            launch_b_scan(bd_, scan_cols_.p, n_cols_, hist_.p, slot_bins_, scale, gp_, d_cand_.p, d_node_tot_.p, 0,
-                          last_wins_ ? 1 : 0, lp, 0u, g_wide_, st_, hist32_, nullptr, colmask(), lw_.child);
+            launch_b_scan(bd_, scan_cols_.p, n_cols_, d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p,
+                          slot_bins_, 1, scale, gp_, d_cand_.p, d_node_tot_.p, 0, last_wins_ ? 1 : 0, lp, 0u,
+                          cfg_.max_leaves, g_wide_, st_, hist32_, nullptr, colmask(), lw_.child);
             tm.end();
             launches += 5 + (n_tiles_ ? 1 : 0);  // + replay, partition, copy-back, children, scan
         }

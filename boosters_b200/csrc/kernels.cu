@@ -2227,19 +2227,20 @@ __device__ __forceinline__ float scan_column(Ld ld, const ScanNode& nd, const Sc
     return best.gain;
 }
 
-// One warp: the same for a numeric column of up to 32 SCAN_PER bins at h. The
-// bins are read coalesced and passed through shared memory so that a lane
-// holds SCAN_PER consecutive ones (an odd stride: no bank conflicts): its
-// prefix sums are serial adds and one scan over the lanes, instead of one per
-// 32 bins. Every bin's score is bounded in f32 first; candidates whose score
-// is within 2^-16 of the column's best get their exact gain (the gain is half
-// the score less an offset >= 0, so no other can win or tie; without a bound
-// all do), so the f64 divisions run once or twice per column and warp instead
-// of 8 to 16 times. 1M x 100, depth 8: the searches of a q8 tree 130 us, before
-// 158; of an fp32 tree 156, before 175; a level of few nodes 11.5, before 14
-// (half of it the hand-off to the last block and its decisions).
+// One warp: the same for a numeric column of up to 32 SCAN_PER bins whose sums
+// lie in the warp's shared scratch `buf`, in order and zero from n_bins on (the
+// caller has made the stores visible to the warp). A lane takes SCAN_PER
+// consecutive bins (an odd stride: no bank conflicts): its prefix sums are
+// serial adds and one scan over the lanes, instead of one per 32 bins. Every
+// bin's score is bounded in f32 first; candidates whose score is within 2^-16
+// of the column's best get their exact gain (the gain is half the score less an
+// offset >= 0, so no other can win or tie; without a bound all do), so the f64
+// divisions run once or twice per column and warp instead of 8 to 16 times.
+// 1M x 100, depth 8: the searches of a q8 tree 130 us, before 158; of an fp32
+// tree 156, before 175; a level of few nodes 11.5, before 14 (half of it the
+// hand-off to the last block and its decisions).
 template <typename HB>
-__device__ __forceinline__ float scan_numeric(const HB* h, const ScanNode& nd, const ScanColumn& cm, const ScanUnits& un,
+__device__ __forceinline__ float scan_numeric(const ScanNode& nd, const ScanColumn& cm, const ScanUnits& un,
                                               const GainParamsDev& gp, ColCand* out, long long* tot, HB* buf,
                                               bool masked) {
     using Acc = decltype(HB{}.g);
@@ -2249,19 +2250,7 @@ __device__ __forceinline__ float scan_numeric(const HB* h, const ScanNode& nd, c
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nb = cm.n_bins, pc = nd.count;
     T2* row = reinterpret_cast<T2*>(buf);
-    {
-        T2 v[SCAN_PER];
-#pragma unroll
-        for (uint32_t q = 0; q < SCAN_PER; ++q) {
-            const uint32_t b = q * 32u + lane;
-            v[q].x = v[q].y = 0;
-            if (b < nb) v[q] = reinterpret_cast<const T2*>(h)[b];
-        }
-#pragma unroll
-        for (uint32_t q = 0; q < SCAN_PER; ++q) row[q * 32u + lane] = v[q];
-    }
     const double ig = un.ig, ih = un.ih;
-    __syncwarp();
     T2 P[SCAN_PER];
     Acc sg = 0, sh = 0;
 #pragma unroll
@@ -2362,15 +2351,32 @@ __device__ __forceinline__ float scan_numeric(const HB* h, const ScanNode& nd, c
 // warp's scan_scratch<HB>() bytes.
 template <typename HB>
 __device__ float scan_item(const ScanNode& nd, const ScanColumn& cm, uint32_t node, uint32_t col, uint32_t n_cols,
-                           const HB* __restrict__ hist, uint64_t slot_bins, const double* __restrict__ scale,
+                           const HB* hist, uint64_t slot_bins, const double* __restrict__ scale,
                            const ScanUnits& un, const GainParamsDev& gp, ColCand* __restrict__ cand,
                            long long* __restrict__ node_tot, unsigned char* scratch, const uint8_t* __restrict__ cmask) {
     const HB* h = hist + (size_t)nd.slot * slot_bins + cm.hist_off;
     ColCand* out = cand + (size_t)node * n_cols + col;
     long long* tot = col == 0 ? node_tot + 2 * node : nullptr;
     const bool masked = cmask && !cmask[col];
-    if (!cm.is_cat && cm.n_bins <= 32u * SCAN_PER && cm.n_bins)
-        return scan_numeric<HB>(h, nd, cm, un, gp, out, tot, reinterpret_cast<HB*>(scratch), masked);
+    if (!cm.is_cat && cm.n_bins <= 32u * SCAN_PER && cm.n_bins) {
+        // read coalesced, staged in shared memory
+        struct alignas(sizeof(HB)) Raw {
+            decltype(HB{}.g) x, y;
+        };
+        Raw v[SCAN_PER];
+        Raw* row = reinterpret_cast<Raw*>(scratch);
+        const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+        for (uint32_t q = 0; q < SCAN_PER; ++q) {
+            const uint32_t b = q * 32u + lane;
+            v[q].x = v[q].y = 0;
+            if (b < cm.n_bins) v[q] = reinterpret_cast<const Raw*>(h)[b];
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < SCAN_PER; ++q) row[q * 32u + lane] = v[q];
+        __syncwarp();
+        return scan_numeric<HB>(nd, cm, un, gp, out, tot, reinterpret_cast<HB*>(scratch), masked);
+    }
     return scan_column<HB>([h](uint32_t b) { return h[b]; }, nd, cm, scale, gp, out, tot,
                            reinterpret_cast<double*>(scratch), reinterpret_cast<uint32_t*>(scratch + SORT_N * 8), masked);
 }
@@ -4036,34 +4042,151 @@ __device__ __forceinline__ unsigned long long cand_key(float g, uint32_t col, in
     return ((unsigned long long)u << 32) | (last_wins ? col : ~col);
 }
 
-// Split finding of every node of the level (two children per expanding
-// node) and the reduction over columns: each (node, column) warp posts its
-// candidate's key to d.node_key[node]; the last block turns the winners into
-// frontier b's splits (the winner's full candidate from cand), resets the
-// keys, and derives the next level's decisions (rows in buffer buf).
-template <typename HB>
-__global__ void __launch_bounds__(SCAN_WARPS * 32, 3)
-k_b_scan(BDev d, const ScanColumn* __restrict__ cols, uint32_t n_cols, const HB* __restrict__ hist,
-         uint64_t slot_bins, const double* __restrict__ scale, GainParamsDev gp, ColCand* __restrict__ cand,
+// The G warps of a column group wait for one another (G * 32 threads; the
+// groups of a block have barriers of their own).
+template <int G>
+__device__ __forceinline__ void group_sync(uint32_t grp) {
+    if (G == SCAN_WARPS)
+        __syncthreads();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(grp + 1u), "n"(G * 32) : "memory");
+}
+
+// Split finding of a level's nodes (two children per expanding node) from the
+// row segments' partial histograms, and the reduction over columns. GS x GB
+// warps take one column of one expanding node: warp w sums every GS-th
+// segment's partials of every GB-th 32 bins; the group adds the shared rows of
+// its GS segment shares to the smaller child's sums, derives the sibling's from
+// the parent's histogram (exact integers, as k_b_merge), stores both children's
+// unless no later level reads them (store == 0), and warps 0 and 1 search the
+// two children's splits from shared memory. Columns whose sums are merged
+// already (col_part null, or 0xFFFFFFFF: a general tile's) are searched from
+// memory. Each search posts its candidate's key to d.node_key[node]; the last
+// block turns the winners into frontier b's splits (the winner's full candidate
+// from cand), resets the keys, and derives the next level's decisions (rows in
+// buffer buf).
+// Bound by the dependent loads of a column (facts, partials, parent) and, on
+// deep levels, by issue slots (half are used); the merged histograms are not
+// read back and the last level's not written. Merge and search of a 1M x 100,
+// depth 8 tree: q8 207 us as two kernels a level, 177 as one; fp32 268 and 244;
+// 8 nodes of 50 columns 16.8 and 14.9. Blocks: two an SM where more registers
+// hold more loads (a third spills: 32.6 us for 27.2 at 32 nodes, fp32).
+template <typename E, typename HB, int GS, int GB>
+__global__ void __launch_bounds__(SCAN_WARPS * 32, GS * GB == 2 && sizeof(HB) == 8 ? 3 : 2)
+k_b_scan(BDev d, const ScanColumn* __restrict__ cols, uint32_t n_cols, const uint32_t* __restrict__ col_part,
+         const E* __restrict__ part, uint32_t n_tiles, HB* __restrict__ hist, uint64_t slot_bins, int store,
+         const double* __restrict__ scale, GainParamsDev gp, ColCand* __restrict__ cand,
          long long* __restrict__ node_tot, int b, int last_wins, LeafParams lp, uint32_t buf,
          const ScanNode* __restrict__ root, const uint8_t* __restrict__ colmask, NodeSplit* __restrict__ lw_out) {
     BST_PDL_ENTER();
+    using Acc = decltype(HB{}.g);
+    struct alignas(sizeof(HB)) T2 {
+        Acc x, y;
+    };
     __shared__ __align__(16) unsigned char scratch[SCAN_WARPS][scan_scratch<HB>()];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t n_nodes = root ? 1u : 2 * d.state->n_exp;
-    const uint32_t col_blocks = (n_cols + SCAN_WARPS - 1) / SCAN_WARPS;
-    const uint64_t items = (uint64_t)n_nodes * col_blocks;
-    if (blockIdx.x < items) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    constexpr int G = GS * GB, UN = sizeof(E) == 8 ? (GS == 8 ? 3 : 4) : 2;
+    const uint32_t grp = warp / G, w = warp % G;
+    const uint32_t n_exp = d.state->n_exp, n_seg = d.state->hist_chunks;
+    const uint32_t n_nodes = root ? 1u : 2 * n_exp;
+    const uint64_t units = (uint64_t)(root ? 1u : n_exp) * n_cols;
+    const uint64_t u0 = (uint64_t)blockIdx.x * (SCAN_WARPS / G) + grp;
+    if (u0 < units) {
         const ScanUnits un(scale, gp);
-        for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
-            const uint32_t node = (uint32_t)(it / col_blocks);
-            const uint32_t col = (uint32_t)(it % col_blocks) * SCAN_WARPS + warp;
-            if (col < n_cols) {
+        const size_t rec = (size_t)n_tiles * LANE_PART_STRIDE;
+        T2* row = reinterpret_cast<T2*>(scratch[grp * G]);  // the group's rows follow one another
+        constexpr uint32_t RS = scan_scratch<HB>() / sizeof(T2);
+        static_assert(scan_scratch<HB>() % sizeof(T2) == 0, "rows of whole entries");
+        for (uint64_t u = u0; u < units; u += (uint64_t)gridDim.x * (SCAN_WARPS / G)) {
+            const uint32_t j = (uint32_t)(u / n_cols), col = (uint32_t)(u % n_cols);
+            const ScanColumn cm = cols[col];
+            const uint32_t cp = col_part ? col_part[col] : 0xFFFFFFFFu;
+            const uint32_t left = d.exp[j].left_pnode, right = d.exp[j].right_pnode;
+            const uint32_t lc = d.exp[j].lc, rc = d.exp[j].rc;
+            const uint32_t c0 = d.exp[j].hist_off, c1 = j + 1 < n_exp ? d.exp[j + 1].hist_off : n_seg;
+            if (cp != 0xFFFFFFFFu) {  // <= LANE_ROWS bins
+                constexpr uint32_t KB = (SCAN_PER + GB - 1) / GB, KR = (SCAN_PER + G - 1) / G;
+                const E* p = part + (size_t)(cp >> 16) * LANE_PART_STRIDE + (cp & 0xFFFFu);
+                T2* L = reinterpret_cast<T2*>(hist) + (size_t)left * slot_bins + cm.hist_off;
+                T2* R = reinterpret_cast<T2*>(hist) + (size_t)right * slot_bins + cm.hist_off;
+                T2 par[KR];  // the parent's sums of the bins this thread finishes
+#pragma unroll
+                for (uint32_t k = 0; k < KR; ++k) {
+                    const uint32_t i = (k * G + w) * 32u + lane;
+                    par[k].x = par[k].y = 0;
+                    if (!root && i < cm.n_bins) par[k] = L[i];
+                }
+                T2 a[KB];
+#pragma unroll
+                for (uint32_t k = 0; k < KB; ++k) a[k].x = a[k].y = 0;
+#pragma unroll(UN)
+                for (uint32_t c = c0 + w / GB; c < c1; c += GS) {
+                    E v[KB];
+#pragma unroll
+                    for (uint32_t k = 0; k < KB; ++k) {
+                        const uint32_t i = (k * GB + w % GB) * 32u + lane;
+                        v[k].x = v[k].y = 0;
+                        if (i < cm.n_bins) v[k] = p[(size_t)c * rec + i];
+                    }
+#pragma unroll
+                    for (uint32_t k = 0; k < KB; ++k) {
+                        a[k].x += (Acc)v[k].x;
+                        a[k].y += (Acc)v[k].y;
+                    }
+                }
+                if (GS > 1) {
+#pragma unroll
+                    for (uint32_t k = 0; k < KB; ++k) {
+                        const uint32_t i = (k * GB + w % GB) * 32u + lane;
+                        if (i < 32u * SCAN_PER) row[(w / GB) * RS + i] = a[k];
+                    }
+                    group_sync<G>(grp);
+                }
+                const bool st = store || cm.is_cat;  // categorical columns are searched from memory
+                const bool left_small = lc <= rc;    // grower.rs:398-402
+#pragma unroll
+                for (uint32_t k = 0; k < KR; ++k) {
+                    const uint32_t i = (k * G + w) * 32u + lane;
+                    if (i >= 32u * SCAN_PER) continue;
+                    T2 s;
+                    if (GS > 1) {
+                        s = row[i];
+#pragma unroll
+                        for (uint32_t q = 1; q < GS; ++q) {
+                            s.x += row[q * RS + i].x;
+                            s.y += row[q * RS + i].y;
+                        }
+                    } else {
+                        s = a[k];
+                    }
+                    T2 o;
+                    o.x = par[k].x - s.x;
+                    o.y = par[k].y - s.y;
+                    const T2 r = root || !left_small ? s : o, l = left_small ? s : o;
+                    row[i] = root ? s : l;
+                    row[RS + i] = r;
+                    if (st && i < cm.n_bins) {
+                        if (!root) L[i] = l;
+                        R[i] = r;
+                    }
+                }
+                group_sync<G>(grp);
+            }
+            if (w < (root ? 1u : 2u)) {
+                const uint32_t node = root ? 0u : 2 * j + w;
                 const ScanNode nd = root ? root[0] : d.scan_nodes[node];
-                const float g = scan_item(nd, cols[col], node, col, n_cols, hist, slot_bins, scale, un, gp, cand, node_tot,
-                                          scratch[warp], colmask ? colmask + (size_t)nd.pad * n_cols : nullptr);
+                const uint8_t* cmask = colmask ? colmask + (size_t)nd.pad * n_cols : nullptr;
+                float g;
+                if (cp != 0xFFFFFFFFu && !cm.is_cat)
+                    g = scan_numeric<HB>(nd, cm, un, gp, cand + (size_t)node * n_cols + col,
+                                         col == 0 ? node_tot + 2 * node : nullptr,
+                                         reinterpret_cast<HB*>(row + w * RS), cmask && !cmask[col]);
+                else
+                    g = scan_item(nd, cm, node, col, n_cols, hist, slot_bins, scale, un, gp, cand, node_tot,
+                                  reinterpret_cast<unsigned char*>(row + w * RS), cmask);
                 if (lane == 0 && g > -INFINITY) atomicMax(&d.node_key[node], cand_key(g, col, last_wins));
             }
+            group_sync<G>(grp);  // the rows are free for the next column
         }
     }
     if (!last_block(d.state)) return;
@@ -4106,20 +4229,48 @@ k_b_scan(BDev d, const ScanColumn* __restrict__ cols, uint32_t n_cols, const HB*
     decide_body(d, b, lp, scale, buf);
 }
 
-uint32_t scan_col_blocks(uint32_t n_cols) { return (n_cols + SCAN_WARPS - 1) / SCAN_WARPS; }
+template <typename E, typename HB>
+static void launch_b_scan_t(const BDev& d, const ScanColumn* cols, uint32_t n_cols, const uint32_t* col_part,
+                            const void* part, uint32_t n_tiles, HB* hist, uint64_t slot_bins, int store,
+                            const double* scale, GainParamsDev gp, ColCand* cand, long long* node_tot, int b,
+                            int last_wins, LeafParams lp, uint32_t buf, uint32_t max_exp, uint32_t max_grid,
+                            cudaStream_t st, const ScanNode* root, const uint8_t* colmask, NodeSplit* lw_out) {
+    // warps per column and node: as many as the chip holds at 16 an SM, in three
+    // shapes; deeper levels have few segments a node, so their two warps share
+    // the bins (at 4 nodes of 100 columns, q8: 21.3 us with eight warps a
+    // column, in two waves, 16.9 with four; at 16 nodes 23 with two sharing the
+    // segments, 20 the bins)
+    const uint64_t units = (uint64_t)max_exp * n_cols, room = (uint64_t)sm_count() * 16u;
+    auto go = [&](auto k, uint32_t G) {
+        const uint64_t blocks = (units * G + SCAN_WARPS - 1) / SCAN_WARPS;
+        launch_k(k, (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(max_grid, blocks)), SCAN_WARPS * 32, 0, st, d, cols,
+                 n_cols, col_part, static_cast<const E*>(part), n_tiles, hist, slot_bins, store, scale, gp, cand, node_tot,
+                 b, last_wins, lp, buf, root, colmask, lw_out);
+    };
+    if (units * 8u <= room)
+        go(k_b_scan<E, HB, 8, 1>, 8);
+    else if (units * 4u <= room)
+        go(k_b_scan<E, HB, 2, 2>, 4);
+    else
+        go(k_b_scan<E, HB, 1, 2>, 2);
+}
 
-void launch_b_scan(const BDev& d, const ScanColumn* cols, uint32_t n_cols, const void* hist, uint64_t slot_bins,
-                   const double* scale, GainParamsDev gp, ColCand* cand, long long* node_tot, int b, int last_wins,
-                   LeafParams lp, uint32_t buf, uint32_t grid, cudaStream_t st, int hist32, const ScanNode* root,
+void launch_b_scan(const BDev& d, const ScanColumn* cols, uint32_t n_cols, const uint32_t* col_part, const void* part,
+                   uint32_t n_tiles, int mode, void* hist, uint64_t slot_bins, int store, const double* scale,
+                   GainParamsDev gp, ColCand* cand, long long* node_tot, int b, int last_wins, LeafParams lp,
+                   uint32_t buf, uint32_t max_exp, uint32_t max_grid, cudaStream_t st, int hist32, const ScanNode* root,
                    const uint8_t* colmask, NodeSplit* lw_out) {
     if (hist32)
-        launch_k(k_b_scan<HBin32>, grid, SCAN_WARPS * 32, 0, st, d, cols, n_cols, static_cast<const HBin32*>(hist), slot_bins,
-                                                           scale, gp, cand, node_tot, b, last_wins, lp, buf, root,
-                                                           colmask, lw_out);
+        launch_b_scan_t<int2>(d, cols, n_cols, col_part, part, n_tiles, static_cast<HBin32*>(hist), slot_bins, store,
+                              scale, gp, cand, node_tot, b, last_wins, lp, buf, max_exp, max_grid, st, root, colmask,
+                              lw_out);
+    else if (mode == GRAD_F32)
+        launch_b_scan_t<longlong2>(d, cols, n_cols, col_part, part, n_tiles, static_cast<HBin*>(hist), slot_bins, store,
+                                   scale, gp, cand, node_tot, b, last_wins, lp, buf, max_exp, max_grid, st, root,
+                                   colmask, lw_out);
     else
-        launch_k(k_b_scan<HBin>, grid, SCAN_WARPS * 32, 0, st, d, cols, n_cols, static_cast<const HBin*>(hist), slot_bins,
-                                                         scale, gp, cand, node_tot, b, last_wins, lp, buf, root,
-                                                         colmask, lw_out);
+        launch_b_scan_t<int2>(d, cols, n_cols, col_part, part, n_tiles, static_cast<HBin*>(hist), slot_bins, store, scale,
+                              gp, cand, node_tot, b, last_wins, lp, buf, max_exp, max_grid, st, root, colmask, lw_out);
 }
 
 // This thread's share of the fixed-point sums of positions [start, start +

@@ -506,26 +506,29 @@ void launch_b_merge(const BDev& d, void* hist, uint64_t slot_bins, uint32_t tota
 constexpr uint32_t LW_K_FROM_STATE = 0xFFFFFFFFu;
 void launch_lw_children(const BDev& d, const PartWork* pw, const unsigned* cursors, uint32_t k, ScanNode* scan_nodes,
                         const unsigned* scnt, cudaStream_t st);
-// split finding of the level's nodes and the reduction over columns into
-// frontier b, then (last block) the decisions of the next level, whose rows
-// are in buffer buf
+// the merge of the level's partials (part, as launch_b_merge; col_part
+// [n_cols]: a column's tile << 16 | offset in the tile's partial record, or
+// 0xFFFFFFFF: a general tile's, whose sums launch_b_merge has merged), split
+// finding of the level's nodes and the reduction over columns into frontier b,
+// then (last block) the decisions of the next level, whose rows are in buffer
+// buf
+// store 0: no later level reads these nodes' histograms
+// max_exp: expanding nodes of the level at most
 // root (or null): the level is the root alone, described by *root (rows in
 // buffer 0, frontier 0); colmask (or null): the level's column masks, a
 // node's row chosen by ScanNode.pad (0 for the device-built levels)
 // lw_out (or null): leaf-wise steps: the last block writes the 2 n_exp
 // children's splits there instead of a frontier and takes no decisions
-void launch_b_scan(const BDev& d, const ScanColumn* cols, uint32_t n_cols, const void* hist,
-                   uint64_t slot_bins, const double* scale, GainParamsDev gp, ColCand* cand,
-                   long long* node_tot, int b, int last_wins, LeafParams lp, uint32_t buf, uint32_t grid,
-                   cudaStream_t st, int hist32 = 0, const ScanNode* root = nullptr,
-                   const uint8_t* colmask = nullptr, NodeSplit* lw_out = nullptr);
+void launch_b_scan(const BDev& d, const ScanColumn* cols, uint32_t n_cols, const uint32_t* col_part, const void* part,
+                   uint32_t n_tiles, int mode, void* hist, uint64_t slot_bins, int store, const double* scale,
+                   GainParamsDev gp, ColCand* cand, long long* node_tot, int b, int last_wins, LeafParams lp,
+                   uint32_t buf, uint32_t max_exp, uint32_t max_grid, cudaStream_t st, int hist32 = 0,
+                   const ScanNode* root = nullptr, const uint8_t* colmask = nullptr, NodeSplit* lw_out = nullptr);
 // last level: the smaller children's sums, then (last block) both children's
 // sums into frontier b and, when `finalize`, the tree's leaves from frontier b
 // as launch_b_finalize(d, b, lp, scale, buf) would write them
 void launch_b_sums(const BDev& d, const uint32_t* ridx, const GradRef& gr, int b, uint32_t grid, cudaStream_t st,
                    int finalize, LeafParams lp, const double* scale, uint32_t buf);
-// work items of k_b_scan per node (column blocks of its warps)
-uint32_t scan_col_blocks(uint32_t n_cols);
 void launch_b_finalize(const BDev& d, int a, LeafParams lp, const double* scale, uint32_t buf, cudaStream_t st);
 // quantised training: exact leaf sums of the f32 gradients (gr: GRAD_F32),
 // then (last block) the leaf values with their fixed-point scale
