@@ -2034,7 +2034,7 @@ class Trainer {
                 // are read again unless their children are leaves
                 launch_b_scan(bd_, scan_cols_.p, n_cols_, d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p,
                               slot_bins_, d + 2 < cfg_.max_depth, scale, gp_, d_cand_.p, d_node_tot_.p, a ^ 1,
-                              last_wins_ ? 1 : 0, lp, (d + 1) & 1u, 1u << std::min(d, 31u), g_wide, st_, hist32_, nullptr,
+                              last_wins_ ? 1 : 0, lp, (d + 1) & 1u, (uint32_t)std::min<uint64_t>(1ull << std::min(d, 31u), d_bexp_.n), g_wide, st_, hist32_, nullptr,
                               colsample_ ? d_colmask_.p + (size_t)(d + 1) * n_cols_ : nullptr);
                 // + column reduction, next level's decisions
                 tm.end();
@@ -2848,7 +2848,7 @@ class Trainer {
             tm.begin(PH_SCAN);
             launch_b_scan(bd_, scan_cols_.p, n_cols_, d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p,
                           slot_bins_, 1, scale, gp_, d_cand_.p, d_node_tot_.p, 0, last_wins_ ? 1 : 0, lp, 0u,
-                          cfg_.max_leaves, g_wide_, st_, hist32_, nullptr, colmask(), lw_.child);
+                          (uint32_t)d_bexp_.n, g_wide_, st_, hist32_, nullptr, colmask(), lw_.child);
             tm.end();
             launches += 5 + (n_tiles_ ? 1 : 0);  // + replay, partition, copy-back, children, scan
         }

@@ -2871,13 +2871,6 @@ __global__ void k_b_root_init(BDev d, uint32_t* __restrict__ ridx, uint64_t n, u
     r.count = (uint32_t)n;
     r.G = 0;
     r.H = 0;
-    r.split.gain = -INFINITY;
-    r.split.col = 0;
-    r.split.bin = 0;
-    r.split.flags = 0;
-    r.split.cats[0] = r.split.cats[1] = r.split.cats[2] = r.split.cats[3] = 0ull;
-    r.split.tot_g = 0;
-    r.split.tot_h = 0;
     d.front[0][0] = r;
     BExp e;
     e.front = 0;
@@ -2926,39 +2919,93 @@ void launch_b_root_init(const BDev& d, uint32_t* ridx, uint64_t n, uint32_t chun
 // leaves made here keep their rows there).
 constexpr uint32_t DECIDE_THREADS = SCAN_WARPS * 32;  // the block size of its one caller, k_b_scan
 
-__device__ void decide_body(BDev d, int a, LeafParams lp, const double* __restrict__ scale, uint32_t buf) {
+// What decide_body reads that the level's split search does not write, read
+// ahead of the hand-off to the last block (whose own chain of dependent loads
+// is the kernel's tail).
+struct DecidePre {
+    uint4 nd;  // frontier node threadIdx.x: pnode, tnode, begin, count
+    uint32_t n_leaves, n_pnodes, n_tnodes;
+};
+__device__ __forceinline__ DecidePre decide_pre(const BDev& d, int a, uint32_t n_nodes) {
+    DecidePre p;
+    p.nd = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < n_nodes) p.nd = *reinterpret_cast<const uint4*>(&d.front[a][threadIdx.x]);
+    p.n_leaves = d.state->n_leaves;
+    p.n_pnodes = d.state->n_pnodes;
+    p.n_tnodes = d.state->n_tnodes;
+    return p;
+}
+
+// The split search's winner of one node (null: none) and the node's totals;
+// resets the node's key.
+struct Winner {
+    const ColCand* c;
+    uint32_t col;
+    long long G, H;
+};
+__device__ __forceinline__ Winner take_winner(const BDev& d, uint32_t node, const ColCand* cand, const long long* node_tot,
+                                              uint32_t n_cols, int last_wins) {
+    const unsigned long long key = d.node_key[node];
+    Winner v;
+    v.G = node_tot[2 * node];
+    v.H = node_tot[2 * node + 1];
+    d.node_key[node] = 0ull;
+    v.col = last_wins ? (uint32_t)key : ~(uint32_t)key;
+    v.c = key ? cand + (size_t)node * n_cols + v.col : nullptr;
+    return v;
+}
+
+__device__ void decide_body(BDev d, int a, uint32_t nf, const DecidePre& pre, const ColCand* cand,
+                            const long long* node_tot, uint32_t n_cols, int last_wins, LeafParams lp,
+                            const double* __restrict__ scale, uint32_t buf) {
     __shared__ uint32_t sh[66];
     __shared__ uint32_t s_jc[DECIDE_THREADS], s_j[DECIDE_THREADS], s_begin[DECIDE_THREADS];
-    __shared__ uint32_t base_exp, base_leaf, base_chunk, first_right, tn0, nf;
     BState* s = d.state;
-    if (threadIdx.x == 0) {
-        nf = s->n_front;
-        base_exp = 0;
-        base_leaf = s->n_leaves;
-        base_chunk = 0;
-        first_right = s->n_pnodes;
-        tn0 = s->n_tnodes;
-    }
-    __syncthreads();
-    const BNode* A = d.front[a];
+    const uint32_t first_right = pre.n_pnodes, tn0 = pre.n_tnodes;
+    uint32_t base_exp = 0, base_leaf = pre.n_leaves, base_chunk = 0;
+    BNode* A = d.front[a];
     for (uint32_t i0 = 0; i0 < nf; i0 += blockDim.x) {
         const uint32_t i = i0 + threadIdx.x;
         const bool valid = i < nf;
-        BNode nd;
-        if (valid) nd = A[i];
-        const bool ex = valid && (nd.split.flags & 4u) && nd.split.gain > -INFINITY &&
-                        !((double)nd.split.gain <= lp.min_gain);
+        struct {
+            uint32_t pnode, tnode, begin, count;
+            long long G, H;
+        } nd;
+        Winner v;
+        v.c = nullptr;
+        ColCand sp;
+        BColumn bc;
+        sp.gain = -INFINITY;
+        if (valid) {
+            const uint4 q = i0 == 0 ? pre.nd : *reinterpret_cast<const uint4*>(&A[i]);
+            v = take_winner(d, i, cand, node_tot, n_cols, last_wins);
+            nd.pnode = q.x;
+            nd.tnode = q.y;
+            nd.begin = q.z;
+            nd.count = q.w;
+            nd.G = v.G;
+            nd.H = v.H;
+            A[i].G = v.G;
+            A[i].H = v.H;
+            if (v.c) {
+                sp.gain = v.c->gain;
+                sp.bin = v.c->bin;
+                sp.flags = v.c->flags;
+                bc = d.bcols[v.col];
+            }
+        }
+        const bool ex = v.c && sp.gain > -INFINITY && !((double)sp.gain <= lp.min_gain);
         const uint32_t nch = ex ? (nd.count + B_PART_CHUNK - 1) / B_PART_CHUNK : 0u;
         uint32_t te, tc, je, jc;  // expansions and their row chunks in one scan
         block_excl_scan2(ex ? 1u : 0u, nch, sh, &je, &jc, &te, &tc);
         const uint32_t n_tile = min(nf - i0, blockDim.x), tl = n_tile - te, jl = threadIdx.x - je;
         if (valid && !ex) {
-            const float v = leaf_value_dev(nd.G, nd.H, scale, lp);
-            write_leaf(d.tree[nd.tnode], nd.G, nd.H, scale, v);
+            const float lv = leaf_value_dev(nd.G, nd.H, scale, lp);
+            write_leaf(d.tree[nd.tnode], nd.G, nd.H, scale, lv);
             BLeaf lf;
             lf.begin = nd.begin;
             lf.count = nd.count;
-            lf.value = v;
+            lf.value = lv;
             lf.tnode = nd.tnode;
             lf.chunk_off = 0;
             lf.buf = buf;
@@ -2967,20 +3014,18 @@ __device__ void decide_body(BDev d, int a, LeafParams lp, const double* __restri
         if (ex) {
             const uint32_t j = base_exp + je;
             const uint32_t tla = tn0 + 2 * j, tra = tn0 + 2 * j + 1;
-            const bool cat = (nd.split.flags & 2u) != 0;
-            const uint32_t col = nd.split.col;
-            const BColumn bc = d.bcols[col];
+            const bool cat = (sp.flags & 2u) != 0;
             BTreeNode t;
-            t.col = col;
-            t.bin = nd.split.bin;
-            t.flags = (nd.split.flags & 1u) | (cat ? 2u : 0u);
+            t.col = v.col;
+            t.bin = sp.bin;
+            t.flags = (sp.flags & 1u) | (cat ? 2u : 0u);
             t.left = tla;
             t.right = tra;
-            t.gain = nd.split.gain;
+            t.gain = sp.gain;
             t.leaf = 0.0f;
             t.G = (double)nd.G * scale[2];
             t.H = (double)nd.H * scale[3];
-            for (int q = 0; q < 4; ++q) t.cats[q] = nd.split.cats[q];
+            for (int q = 0; q < 4; ++q) t.cats[q] = v.c->cats[q];
             d.tree[nd.tnode] = t;
             BExp e;
             e.front = i;
@@ -2998,11 +3043,11 @@ __device__ void decide_body(BDev d, int a, LeafParams lp, const double* __restri
             w.count = nd.count;
             w.matrix = bc.matrix;
             w.pos = bc.pos;
-            w.thr_bin = nd.split.bin;
-            w.flags = (nd.split.flags & 1u) | (bc.has_missing ? 2u : 0u) | (cat ? 4u : 0u);
+            w.thr_bin = sp.bin;
+            w.flags = (sp.flags & 1u) | (bc.has_missing ? 2u : 0u) | (cat ? 4u : 0u);
             w.default_bin = bc.default_bin;
             w.pad = 0;
-            for (int q = 0; q < 4; ++q) w.cats[q] = nd.split.cats[q];
+            for (int q = 0; q < 4; ++q) w.cats[q] = t.cats[q];
             d.pworks[j] = w;
             d.cursors[2 * j] = nd.begin;
             d.cursors[2 * j + 1] = nd.begin + nd.count;
@@ -3028,13 +3073,10 @@ __device__ void decide_body(BDev d, int a, LeafParams lp, const double* __restri
             const uint32_t g = base_chunk + c;
             if (g < d.max_part_chunks) d.part_map[g] = make_uint2(s_j[lo], s_begin[lo] + (c - s_jc[lo]) * B_PART_CHUNK);
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            base_exp += te;
-            base_leaf += tl;
-            base_chunk += tc;
-        }
-        __syncthreads();
+        __syncthreads();  // s_jc / s_j / s_begin are reused by the next tile
+        base_exp += te;
+        base_leaf += tl;
+        base_chunk += tc;
     }
     if (threadIdx.x == 0) {
         s->n_exp = base_exp;
@@ -3064,23 +3106,39 @@ __device__ bool last_block(BState* s) {
     return last;
 }
 
-__device__ void children_body(BDev d, int a, int need_split);
+// What children_body reads of expansion threadIdx.x, read ahead of the hand-off
+// to the last block (whose own chain of dependent loads is the kernel's tail;
+// this and decide_body's: a 1M x 100 depth-8 tree 681 -> 672 us in q8, 882 ->
+// 874 in fp32, 200K x 50 322 -> 318).
+struct ChildPre {
+    uint32_t n_exp;
+    BExp e;
+    uint4 nd;  // the expanding node's pnode, tnode, begin, count
+};
+__device__ void children_body(BDev d, int a, int need_split, const ChildPre& pre);
 
 // Partition of every expanding node (partition.rs:296-382) over 2048-row
 // chunks (one atomic per side per chunk, part_rows) from row-index buffer
 // rin into rout; the last block then derives the children (children_body).
+// Four blocks an SM: the 490 chunks of 1M rows run in one wave (three: 20.8
+// instead of 15.8 us).
 template <typename Q>
-__global__ void __launch_bounds__(PART_THREADS)
+__global__ void __launch_bounds__(PART_THREADS, 4)
 k_b_partition(BDev d, const uint32_t* __restrict__ ridx, uint32_t* __restrict__ tmp,
               const uint8_t* __restrict__ bins8, uint32_t s8, const uint16_t* __restrict__ bins16, uint32_t s16,
               int a, int need_split, const Q* __restrict__ qin, Q* __restrict__ qout, BinsFM fm) {
     BST_PDL_ENTER();
     __shared__ PartWork w;
     __shared__ uint2 s_m;
+    uint2 m0 = make_uint2(0u, 0u);  // the first chunk's facts, read before the level's chunk count is here
+    if (threadIdx.x == 0 && blockIdx.x < d.max_part_chunks) m0 = d.part_map[blockIdx.x];
     const uint32_t total = min(d.state->part_chunks, d.max_part_chunks);
+    ChildPre pre;
+    pre.n_exp = d.state->n_exp;
+    const uint32_t front = threadIdx.x < pre.n_exp ? d.exp[threadIdx.x].front : 0u;
     for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
         if (threadIdx.x == 0) {
-            const uint2 m = d.part_map[c];  // (expansion, first row)
+            const uint2 m = c == blockIdx.x ? m0 : d.part_map[c];  // (expansion, first row)
             s_m = m;
             w = d.pworks[m.x];
         }
@@ -3095,7 +3153,11 @@ k_b_partition(BDev d, const uint32_t* __restrict__ ridx, uint32_t* __restrict__ 
         part_rows<Q>(w, start, len, d.cursors + 2 * j, ridx, tmp, bins8, s8, bins16, s16, qin, qout, fm.b8, fm.b16,
                      fm.n, d.rmask, d.rmask ? d.scnt + 2 * j : nullptr);
     }
-    if (last_block(d.state)) children_body(d, a, need_split);
+    if (threadIdx.x < pre.n_exp) {
+        pre.e = d.exp[threadIdx.x];
+        pre.nd = *reinterpret_cast<const uint4*>(&d.front[a][front]);
+    }
+    if (last_block(d.state)) children_body(d, a, need_split, pre);
 }
 
 void launch_b_partition(const BDev& d, const uint32_t* rin, uint32_t* rout, const uint8_t* bins8, uint32_t s8,
@@ -3210,23 +3272,17 @@ __device__ __forceinline__ uint32_t level_chunk(const BDev& d, unsigned long lon
     return (uint32_t)(want < 1024ull ? 1024ull : (want > d.hist_seg_max ? d.hist_seg_max : want));
 }
 
-__device__ void children_body(BDev d, int a, int need_split) {
+__device__ void children_body(BDev d, int a, int need_split, const ChildPre& pre) {
     __shared__ uint32_t sh[66];
     __shared__ uint32_t s_jc[PART_THREADS], s_own[PART_THREADS];  // block size of its caller, k_b_partition
-    __shared__ uint32_t base, s_exp;
+    __shared__ uint32_t base;
     BState* s = d.state;
-    if (threadIdx.x == 0) {
-        s_exp = s->n_exp;
-        base = 0;
-    }
-    __syncthreads();
-    const uint32_t n_exp = s_exp;
+    if (threadIdx.x == 0) base = 0;
+    const uint32_t n_exp = pre.n_exp;
     const BNode* A = d.front[a];
     BNode* B = d.front[a ^ 1];
     // the children of expansion j (all but its hist_off)
-    auto child = [&](uint32_t j) {
-        BExp e = d.exp[j];
-        const uint4 nd = *reinterpret_cast<const uint4*>(&A[e.front]);  // pnode, tnode, begin, count
+    auto child = [&](uint32_t j, BExp e, const uint4& nd) {
         const uint32_t lc = d.cursors[2 * j] - nd.z, rc = nd.w - lc;
         const bool left_small = lc <= rc;
         e.lc = lc;
@@ -3243,12 +3299,6 @@ __device__ void children_body(BDev d, int a, int need_split) {
         r.begin = nd.z + lc;
         r.count = rc;
         l.G = l.H = r.G = r.H = 0;
-        l.split.gain = r.split.gain = -INFINITY;
-        l.split.col = r.split.col = 0;
-        l.split.bin = r.split.bin = 0;
-        l.split.flags = r.split.flags = 0;
-        for (int q = 0; q < 4; ++q) l.split.cats[q] = r.split.cats[q] = 0ull;
-        l.split.tot_g = l.split.tot_h = r.split.tot_g = r.split.tot_h = 0;
         B[2 * j] = l;
         B[2 * j + 1] = r;
         // row sampling: the split search counts the sampled rows
@@ -3264,7 +3314,7 @@ __device__ void children_body(BDev d, int a, int need_split) {
         const bool valid = j < n_exp;
         BExp e;
         e.small_count = 0;
-        if (valid) e = child(j);
+        if (valid) e = child(j, pre.e, pre.nd);
         uint32_t x0, x1, t0, t1;
         block_excl_scan2(e.small_count, 0u, sh, &x0, &x1, &t0, &t1);  // rows fit 32 bits
         rows = t0;
@@ -3283,7 +3333,8 @@ __device__ void children_body(BDev d, int a, int need_split) {
         if (threadIdx.x == 0) s_rows = 0ull;
         __syncthreads();
         for (uint32_t j = threadIdx.x; j < n_exp; j += blockDim.x) {
-            const BExp e = child(j);
+            const BExp e0 = d.exp[j];
+            const BExp e = child(j, e0, *reinterpret_cast<const uint4*>(&A[e0.front]));
             d.exp[j] = e;
             atomicAdd(&s_rows, (unsigned long long)e.small_count);
         }
@@ -4089,8 +4140,8 @@ k_b_scan(BDev d, const ScanColumn* __restrict__ cols, uint32_t n_cols, const uin
     const uint32_t grp = warp / G, w = warp % G;
     const uint32_t n_exp = d.state->n_exp, n_seg = d.state->hist_chunks;
     const uint32_t n_nodes = root ? 1u : 2 * n_exp;
-    const uint64_t units = (uint64_t)(root ? 1u : n_exp) * n_cols;
     const uint64_t u0 = (uint64_t)blockIdx.x * (SCAN_WARPS / G) + grp;
+    const uint64_t units = (uint64_t)(root ? 1u : n_exp) * n_cols;
     if (u0 < units) {
         const ScanUnits un(scale, gp);
         const size_t rec = (size_t)n_tiles * LANE_PART_STRIDE;
@@ -4189,44 +4240,27 @@ k_b_scan(BDev d, const ScanColumn* __restrict__ cols, uint32_t n_cols, const uin
             group_sync<G>(grp);  // the rows are free for the next column
         }
     }
+    DecidePre pre;
+    if (!lw_out) pre = decide_pre(d, b, n_nodes);
     if (!last_block(d.state)) return;
-    BNode* B = d.front[b];
-    // the winner of one node: its split, the key reset
-    auto winner = [&](uint32_t node) {
-        const unsigned long long key = d.node_key[node];
-        NodeSplit sp;
-        sp.tot_g = node_tot[2 * node];
-        sp.tot_h = node_tot[2 * node + 1];
-        d.node_key[node] = 0ull;
-        if (key == 0ull) {
-            sp.gain = -INFINITY;
-            sp.col = 0;
-            sp.bin = 0;
-            sp.flags = 0;
-            sp.cats[0] = sp.cats[1] = sp.cats[2] = sp.cats[3] = 0ull;
-        } else {
-            const uint32_t col = last_wins ? (uint32_t)key : ~(uint32_t)key;
-            const ColCand& w = cand[(size_t)node * n_cols + col];
-            sp.gain = w.gain;
-            sp.col = col;
-            sp.bin = w.bin;
-            sp.flags = (w.flags & 3u) | 4u;
-            for (int q = 0; q < 4; ++q) sp.cats[q] = w.cats[q];
-        }
-        return sp;
-    };
-    if (lw_out) {
-        for (uint32_t node = threadIdx.x; node < n_nodes; node += blockDim.x) lw_out[node] = winner(node);
-        return;
-    }
+    if (!lw_out) return decide_body(d, b, n_nodes, pre, cand, node_tot, n_cols, last_wins, lp, scale, buf);
     for (uint32_t node = threadIdx.x; node < n_nodes; node += blockDim.x) {
-        const NodeSplit sp = winner(node);
-        B[node].split = sp;
-        B[node].G = sp.tot_g;
-        B[node].H = sp.tot_h;
+        const Winner v = take_winner(d, node, cand, node_tot, n_cols, last_wins);
+        NodeSplit sp;
+        sp.tot_g = v.G;
+        sp.tot_h = v.H;
+        sp.gain = -INFINITY;
+        sp.col = sp.bin = sp.flags = 0;
+        sp.cats[0] = sp.cats[1] = sp.cats[2] = sp.cats[3] = 0ull;
+        if (v.c) {
+            sp.gain = v.c->gain;
+            sp.col = v.col;
+            sp.bin = v.c->bin;
+            sp.flags = (v.c->flags & 3u) | 4u;
+            for (int q = 0; q < 4; ++q) sp.cats[q] = v.c->cats[q];
+        }
+        lw_out[node] = sp;
     }
-    __syncthreads();
-    decide_body(d, b, lp, scale, buf);
 }
 
 template <typename E, typename HB>

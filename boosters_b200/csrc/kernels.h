@@ -305,7 +305,6 @@ struct BColumn {  // per effective column, for decisions and the partition
 struct BNode {  // frontier entry
     uint32_t pnode, tnode, begin, count;
     long long G, H;
-    NodeSplit split;
 };
 struct BTreeNode {  // tree node as grown (training semantics)
     uint32_t col, bin, flags;  // flags: bit0 default_left, bit1 categorical, bit2 leaf
@@ -513,7 +512,7 @@ void launch_lw_children(const BDev& d, const PartWork* pw, const unsigned* curso
 // then (last block) the decisions of the next level, whose rows are in buffer
 // buf
 // store 0: no later level reads these nodes' histograms
-// max_exp: expanding nodes of the level at most
+// max_exp: expanding nodes of the level at most (entries of d.exp)
 // root (or null): the level is the root alone, described by *root (rows in
 // buffer 0, frontier 0); colmask (or null): the level's column masks, a
 // node's row chosen by ScanNode.pad (0 for the device-built levels)

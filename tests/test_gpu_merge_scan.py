@@ -1,9 +1,9 @@
 """The split search that merges the row segments' partial histograms itself,
 against the host-driven levels (a merge kernel, then the search): trees agree
 bit for bit for every number of warps a column gets (few and many columns,
-shallow and deep levels), with columns of the general tiles (more than 264
-bins), categories, missing values, sampling, and a root merged apart (more
-than 128 segments)."""
+shallow levels and ones of more than 256 nodes), with columns of the general
+tiles (more than 264 bins), categories, missing values, sampling, and a root
+merged apart (more than 128 segments)."""
 import numpy as np
 import pytest
 
@@ -25,7 +25,8 @@ def same(tmp_path, ds, **kw):
 
 
 @pytest.mark.parametrize("precision", ["fp32", "q16", "q8"])
-@pytest.mark.parametrize("n,F,depth", [(3000, 1, 1), (20_000, 5, 8), (60_000, 75, 7), (9_000, 310, 5)])
+@pytest.mark.parametrize("n,F,depth", [(3000, 1, 1), (20_000, 5, 8), (60_000, 75, 7), (9_000, 310, 5),
+                                       (40_000, 6, 11)])
 def test_columns_and_levels(tmp_path, precision, n, F, depth):
     x, y = bst.synth.binary(n, F, n_nan_cols=F // 3, seed=F)
     ds = bst.Dataset.from_feature_major(x, y)
