@@ -1948,10 +1948,17 @@ class Trainer {
     // WIDE_MERGE_NODES expanding nodes (the merge splits each node's many row
     // segments over more threads).
     static constexpr uint32_t WIDE_MERGE_NODES = 4;
-    // A root of more segments than this is merged apart: its search has one
-    // block a column, too few to read them (fp32, 245 segments of 100 columns:
-    // merge and search 35 us apart, 41 in one; q8, 62 segments: 18.2 and 18.8).
-    static constexpr uint32_t ROOT_SCAN_SEGS = 128;
+    // Whether the split search merges the partials of nodes of up to `rows` rows
+    // itself. A node of many segments has too few warps a column in the search
+    // to read them, so from SCAN_SEGS (of the largest size) on a merge kernel
+    // goes before it. Merged in the search / apart: the 245 segments of an fp32
+    // root of 1M x 100 41 / 35 us, the 62 of a q8 root 18.8 / 18.2; a tree of
+    // 3M x 60 (366 segments a child) fp32 2.00 / 1.93 ms, leaf-wise 5.98 / 5.82;
+    // of 1M x 100 (122) 0.92 / 0.95, leaf-wise 4.77 / 4.94.
+    static constexpr uint32_t SCAN_SEGS = 128;
+    bool scan_merges(uint64_t rows) const {
+        return (rows + bd_.hist_seg_max - 1) / bd_.hist_seg_max <= SCAN_SEGS;
+    }
     enum class Merge { General, All, AllWide };
     void enqueue_hist(const GradRef& gr, const uint32_t* ridx, bool root, Timer& tm, uint64_t& launches,
                       uint64_t& hist_launches, Merge merge) {
@@ -1996,7 +2003,8 @@ class Trainer {
         launch_b_root_init(bd_, ridx_.p, n_, chunk_rows(n_), st_);  // row ids, root node, root histogram state
         if (n_tiles_) BST_CK(cudaMemsetAsync(hist_.p, 0, hbytes() * slot_bins_, st_));
         tm.end();
-        const bool root_merge = (n_ + chunk_rows(n_) - 1) / chunk_rows(n_) > ROOT_SCAN_SEGS;
+        const bool root_merge = !scan_merges(n_);
+        const bool level_merge = !scan_merges(n_ / 2);  // the smaller children
         enqueue_hist(gh, ridx_.p, true, tm, launches, hist_launches, root_merge ? Merge::AllWide : Merge::General);
         tm.begin(PH_SCAN);
         launch_b_scan(bd_, scan_cols_.p, n_cols_, root_merge ? nullptr : d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p, slot_bins_,
@@ -2028,12 +2036,15 @@ class Trainer {
                     tm.end();
                     launches += 1;
                 }
-                enqueue_hist(gl, rout, false, tm, launches, hist_launches, Merge::General);
+                const Merge merge = !level_merge                                      ? Merge::General
+                                    : (1u << std::min(d, 31u)) <= WIDE_MERGE_NODES ? Merge::AllWide
+                                                                                   : Merge::All;
+                enqueue_hist(gl, rout, false, tm, launches, hist_launches, merge);
                 tm.begin(PH_SCAN);
                 // level d expands at most 2^d nodes; its children's histograms
                 // are read again unless their children are leaves
-                launch_b_scan(bd_, scan_cols_.p, n_cols_, d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p,
-                              slot_bins_, d + 2 < cfg_.max_depth, scale, gp_, d_cand_.p, d_node_tot_.p, a ^ 1,
+                launch_b_scan(bd_, scan_cols_.p, n_cols_, level_merge ? nullptr : d_col_part_.p, d_part_.p,
+                              n_lane_tiles_, qmode_, hist_.p, slot_bins_, d + 2 < cfg_.max_depth, scale, gp_, d_cand_.p, d_node_tot_.p, a ^ 1,
                               last_wins_ ? 1 : 0, lp, (d + 1) & 1u, (uint32_t)std::min<uint64_t>(1ull << std::min(d, 31u), d_bexp_.n), g_wide, st_, hist32_, nullptr,
                               colsample_ ? d_colmask_.p + (size_t)(d + 1) * n_cols_ : nullptr);
                 // + column reduction, next level's decisions
@@ -2093,7 +2104,7 @@ class Trainer {
     // Enqueues the tree of output o into ring slot `si` (no host wait).
     void launch_batched(uint32_t o, uint32_t si) {
         if (use_small_) return launch_small(o, si);
-        BST_RANGE("bst.tree");  // the tree's graph launch (its kernels run after the range closes)
+        BST_RANGE("bst.tree");  // the tree's launches (its kernels run after the range closes)
         Slot& sl = slots_[si];
         const size_t gi = (size_t)o * RING + si;
         sl.timed = false;
@@ -2129,8 +2140,8 @@ class Trainer {
         // the ring lets the host run ahead, so a graph's replay gains nothing
         // (281 and 283 us there, 696 and 698 us a q8 tree of 1M x 100), while
         // capturing and instantiating one, 0.35 ms, came again with every launch
-        // shape explored and for every output (43.5 against 39.4 ms a call of
-        // 50 early-stopped trees).
+        // shape explored and for every output (43.5 against 39.4 ms a call of up
+        // to 60 early-stopped trees).
         if (cfg_.cuda_graph) {
             BST_CK(cudaGraphLaunch(graphs_[gi], st_));
         } else {
@@ -2831,6 +2842,7 @@ class Trainer {
         const double* scale = unit_scale(o);
         launches = 0;
         hist_launches = 0;
+        const bool step_merge = !scan_merges(n_ / 2);
         for (uint32_t k = 0; k < LW_STEPS; ++k) {
             tm.begin(PH_OTHER);
             launch_lw_replay(bd_, lw_, lp, scale, st_);
@@ -2844,10 +2856,10 @@ class Trainer {
                                rowsample_ ? d_scnt_.p : nullptr, st_);
             if (n_tiles_) launch_b_zero_right(bd_, hist_.p, slot_bins_, g_wide_, st_, hist32_);
             tm.end();
-            enqueue_hist(gr, ridx_.p, false, tm, launches, hist_launches, Merge::General);
+            enqueue_hist(gr, ridx_.p, false, tm, launches, hist_launches, step_merge ? Merge::All : Merge::General);
             tm.begin(PH_SCAN);
-            launch_b_scan(bd_, scan_cols_.p, n_cols_, d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p,
-                          slot_bins_, 1, scale, gp_, d_cand_.p, d_node_tot_.p, 0, last_wins_ ? 1 : 0, lp, 0u,
+            launch_b_scan(bd_, scan_cols_.p, n_cols_, step_merge ? nullptr : d_col_part_.p, d_part_.p, n_lane_tiles_,
+                          qmode_, hist_.p, slot_bins_, 1, scale, gp_, d_cand_.p, d_node_tot_.p, 0, last_wins_ ? 1 : 0, lp, 0u,
                           (uint32_t)d_bexp_.n, g_wide_, st_, hist32_, nullptr, colmask(), lw_.child);
             tm.end();
             launches += 5 + (n_tiles_ ? 1 : 0);  // + replay, partition, copy-back, children, scan

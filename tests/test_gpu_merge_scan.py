@@ -2,7 +2,7 @@
 against the host-driven levels (a merge kernel, then the search): trees agree
 bit for bit for every number of warps a column gets (few and many columns,
 shallow levels and ones of more than 256 nodes), with columns of the general
-tiles (more than 264 bins), categories, missing values, sampling, and a root
+tiles (more than 264 bins), categories, missing values, sampling, and nodes
 merged apart (more than 128 segments)."""
 import numpy as np
 import pytest
@@ -46,9 +46,12 @@ def test_wide_columns_categories_sampling(tmp_path, precision, growth):
              precision=precision, colsample_bytree=0.8, subsample=0.8, **kw)
 
 
-@pytest.mark.parametrize("precision", ["fp32", "q8"])
-def test_root_of_many_segments(tmp_path, precision):
-    x, y = bst.synth.regression(560_000, 4, n_informative=4, seed=9)
+# fp32 segments hold 4096 rows: the root alone above 128 of them, then the
+# levels too
+@pytest.mark.parametrize("n", [560_000, 1_100_000])
+@pytest.mark.parametrize("growth", ["depthwise", "leafwise"])
+def test_nodes_of_many_segments(tmp_path, growth, n):
+    x, y = bst.synth.regression(n, 4, n_informative=4, seed=9)
+    kw = dict(growth_strategy=bst.GrowthStrategy.Leafwise, n_leaves=12) if growth == "leafwise" else dict(max_depth=4)
     ds = bst.Dataset.from_feature_major(x, y)
-    same(tmp_path, ds, objective=bst.Objective.squared(), n_estimators=2, max_depth=4, learning_rate=0.3,
-         precision=precision)
+    same(tmp_path, ds, objective=bst.Objective.squared(), n_estimators=2, learning_rate=0.3, precision="fp32", **kw)
