@@ -1516,13 +1516,16 @@ class Trainer {
     }
 
     // ---- small training sets: one cooperative launch per tree (small_tree.cuh) --
-    // us per tree, one launch / level kernels (logistic, depth 6 unless said):
-    // 5,000 x 100 fp32 124 / 263, q8 122 / 248; 50,000 x 100 fp32 249 / 299,
-    // q8 206 / 275, depth 8 430 / 465; 20,000 x 300 (three columns a block)
-    // 371 / 373; 100,000 x 100 fp32 378 / 318, q8 295 / 296. The row loop of
-    // the one launch grows with the rows, so the line is drawn where fp32
-    // crosses.
-    static constexpr uint64_t SMALL_TREE_ROWS = 70000;
+    // us per tree, one launch / level kernels (depth 6 unless said):
+    // 5,000 x 100 fp32 119 / 237; 20,000 x 100 157 / 247; 50,000 x 100 fp32
+    // 230 / 266, q8 194 / 237, depth 8 fp32 374 / 382; 52,000 x 148 234 / 278;
+    // 100,000 x 100 fp32 354 / 279, q8 278 / 259. Few columns leave most blocks
+    // without a row loop while the level kernels get cheaper: 50,000 x 40,
+    // depth 8, 354 / 324; 66,000 x 12, depth 7, 323 / 254. Several columns a
+    // block read the rows again for each: 10,000 x 300, depth 8, 486 / 483;
+    // 25,000 x 200 288 / 279; 20,000 x 300 q8, depth 8, 510 / 407. The lines lie
+    // where the level kernels cross.
+    static constexpr uint64_t SMALL_TREE_ROWS = 28000, SMALL_TREE_ROWS_F32 = 52000, SMALL_TREE_ROWS_Q = 70000;
     bool use_small_ = false;
     DevArray<uint8_t> small_buf_;  // zeroed scratch, then BState and the tree
     DevArray<uint16_t> small_rt_;
@@ -1542,7 +1545,10 @@ class Trainer {
             return false;
         // a block reads every row once per level and column of its own
         const uint64_t per_block = (n_cols_ + sm_count() - 1) / sm_count();
-        if (n_ * per_block > SMALL_TREE_ROWS) return false;
+        const uint64_t rows = per_block > 1 || n_cols_ < sm_count() / 2 ? SMALL_TREE_ROWS
+                              : qmode_ == GRAD_F32                        ? SMALL_TREE_ROWS_F32
+                                                                          : SMALL_TREE_ROWS_Q;
+        if (n_ * per_block > rows) return false;
         uint32_t max_bins = 1;
         bool cat = false;
         for (uint32_t c = 0; c < n_cols_; ++c) {

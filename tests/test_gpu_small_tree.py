@@ -27,15 +27,24 @@ def both(tmp_path, ds, n, record=True, **kw):
     return m
 
 
-# rows below one per block, at warp and block edges, past one 16-bit-sum
-# limit (q16: 65,536); columns below, at and above one per SM; depths 1 to 8
+# rows below one per block, at warp and block edges, near the largest taken for
+# few and for many columns; columns below, at and above one per SM; depths 1 to 8
 @pytest.mark.parametrize("n,F,depth", [(40, 1, 1), (147, 3, 2), (149, 5, 3), (513, 33, 6), (2049, 148, 5),
-                                       (3001, 150, 8), (5000, 100, 6), (66_001, 12, 7)])
+                                       (3001, 150, 8), (5000, 100, 6), (27_900, 12, 7), (51_900, 80, 6)])
 @pytest.mark.parametrize("precision", ["fp32", "q16", "q8"])
 def test_sizes(tmp_path, n, F, depth, precision):
     x, y = bst.synth.regression(n, F, n_informative=min(F, 10), seed=n)
     ds = bst.Dataset.from_feature_major(x, y)
     both(tmp_path, ds, n, objective=bst.Objective.squared(), n_estimators=4, max_depth=depth, learning_rate=0.3,
+         precision=precision)
+
+
+# past one 16-bit-sum limit (q16: 65,536 rows)
+@pytest.mark.parametrize("precision", ["q16", "q8"])
+def test_most_rows(tmp_path, precision):
+    x, y = bst.synth.regression(66_001, 80, n_informative=10, seed=7)
+    ds = bst.Dataset.from_feature_major(x, y)
+    both(tmp_path, ds, 66_001, objective=bst.Objective.squared(), n_estimators=4, max_depth=7, learning_rate=0.3,
          precision=precision)
 
 
