@@ -1954,16 +1954,19 @@ class Trainer {
     // WIDE_MERGE_NODES expanding nodes (the merge splits each node's many row
     // segments over more threads).
     static constexpr uint32_t WIDE_MERGE_NODES = 4;
-    // Whether the split search merges the partials of nodes of up to `rows` rows
-    // itself. A node of many segments has too few warps a column in the search
-    // to read them, so from SCAN_SEGS (of the largest size) on a merge kernel
-    // goes before it. Merged in the search / apart: the 245 segments of an fp32
+    // Whether the split search merges the partials of `nodes` nodes of `rows` rows
+    // in all itself. A node of many segments has too few warps a column in the search
+    // to read them, so above SCAN_SEGS a node a merge kernel goes before
+    // it. Merged in the search / apart: the 245 segments of an fp32
     // root of 1M x 100 41 / 35 us, the 62 of a q8 root 18.8 / 18.2; a tree of
     // 3M x 60 (366 segments a child) fp32 2.00 / 1.93 ms, leaf-wise 5.98 / 5.82;
     // of 1M x 100 (122) 0.92 / 0.95, leaf-wise 4.77 / 4.94.
-    static constexpr uint32_t SCAN_SEGS = 128;
-    bool scan_merges(uint64_t rows) const {
-        return (rows + bd_.hist_seg_max - 1) / bd_.hist_seg_max <= SCAN_SEGS;
+    // 2M x 50, q16, 296 segments of one node: 44 / 30.
+    static constexpr uint64_t SCAN_SEGS = 100;
+    bool scan_merges(uint64_t rows, uint64_t nodes) const {
+        const uint64_t segs = std::max<uint64_t>((rows + bd_.hist_seg_max - 1) / bd_.hist_seg_max,
+                                                 std::min<uint64_t>(bd_.hist_target, rows / 1024));
+        return segs <= SCAN_SEGS * nodes;
     }
     enum class Merge { General, All, AllWide };
     void enqueue_hist(const GradRef& gr, const uint32_t* ridx, bool root, Timer& tm, uint64_t& launches,
@@ -2009,8 +2012,7 @@ class Trainer {
         launch_b_root_init(bd_, ridx_.p, n_, chunk_rows(n_), st_);  // row ids, root node, root histogram state
         if (n_tiles_) BST_CK(cudaMemsetAsync(hist_.p, 0, hbytes() * slot_bins_, st_));
         tm.end();
-        const bool root_merge = !scan_merges(n_);
-        const bool level_merge = !scan_merges(n_ / 2);  // the smaller children
+        const bool root_merge = !scan_merges(n_, 1);
         enqueue_hist(gh, ridx_.p, true, tm, launches, hist_launches, root_merge ? Merge::AllWide : Merge::General);
         tm.begin(PH_SCAN);
         launch_b_scan(bd_, scan_cols_.p, n_cols_, root_merge ? nullptr : d_col_part_.p, d_part_.p, n_lane_tiles_, qmode_, hist_.p, slot_bins_,
@@ -2042,6 +2044,7 @@ class Trainer {
                     tm.end();
                     launches += 1;
                 }
+                const bool level_merge = !scan_merges(n_ / 2, 1ull << std::min(d, 31u));  // the smaller children
                 const Merge merge = !level_merge                                      ? Merge::General
                                     : (1u << std::min(d, 31u)) <= WIDE_MERGE_NODES ? Merge::AllWide
                                                                                    : Merge::All;
@@ -2848,7 +2851,8 @@ class Trainer {
         const double* scale = unit_scale(o);
         launches = 0;
         hist_launches = 0;
-        const bool step_merge = !scan_merges(n_ / 2);
+        // a batch's size is not known here: by segments of the largest size
+        const bool step_merge = n_ / 2 / bd_.hist_seg_max > 128;
         for (uint32_t k = 0; k < LW_STEPS; ++k) {
             tm.begin(PH_OTHER);
             launch_lw_replay(bd_, lw_, lp, scale, st_);

@@ -4281,9 +4281,10 @@ static void launch_b_scan_t(const BDev& d, const ScanColumn* cols, uint32_t n_co
                  n_cols, col_part, static_cast<const E*>(part), n_tiles, hist, slot_bins, store, scale, gp, cand, node_tot,
                  b, last_wins, lp, buf, root, colmask, lw_out);
     };
-    if (units * 8u <= room)
+    // (merged columns need the searching two only)
+    if (col_part && units * 8u <= room)
         go(k_b_scan<E, HB, 8, 1>, 8);
-    else if (units * 4u <= room)
+    else if (col_part && units * 4u <= room)
         go(k_b_scan<E, HB, 2, 2>, 4);
     else
         go(k_b_scan<E, HB, 1, 2>, 2);
