@@ -209,9 +209,15 @@ struct StreamGuard {
 
 // A host array to the device in stream order. Pinned memory: one asynchronous
 // copy. Pageable memory: the driver's own staging runs at 11 GB/s on one
-// thread, so larger arrays go through pinned blocks filled by several threads
-// (120 MB: 10.5 -> 3.9 ms). finish(): the array has been read (the copies may
-// still run); the destructor waits for them.
+// thread, so arrays from MIN_STAGED on go through pinned blocks filled by
+// several threads, one for each PER_THREAD bytes: starting and joining them
+// costs a small copy more than it gains. Host prediction of that many bytes,
+// ms, the driver's copy / 2 / 3 / 4 / 6 threads: 6 MB 0.43 / 0.42 / 0.63 /
+// 0.76 / 0.82; 8 MB 0.52 / 0.42 / 0.80 / 0.82 / 1.1; 16 MB 0.98 / 0.88 / 1.0 /
+// 1.2 / 1.4; 48 MB 3.1 / 2.2 / 1.9 / 2.0 / 2.3; 120 MB 11.3 / 5.6 / 4.2 / 3.8 /
+// 4.0; 400 MB 37.9 / 18.3 / 13.5 / 10.6 / 10.8 (six are faster than four, 12
+// against 14 ms, where the host analyses the table meanwhile). finish(): the
+// array has been read (the copies may still run); the destructor waits for them.
 class HostUpload {
   public:
     HostUpload() = default;
@@ -242,7 +248,7 @@ class HostUpload {
         size_t n = 1;
         if (bytes >= MIN_STAGED) {
             const size_t hw = std::max<size_t>(1, std::thread::hardware_concurrency());
-            n = std::max<size_t>(1, std::min<size_t>({MAX_THREADS, hw / 2, bytes / BLOCK}));
+            n = std::min<size_t>({MAX_THREADS, hw / 2, std::max<size_t>(2, bytes / PER_THREAD)});
         }
         if (n > 1) {
             blocks_.resize(2 * n);
@@ -267,7 +273,8 @@ class HostUpload {
     }
 
   private:
-    static constexpr size_t BLOCK = (size_t)1 << 20, MIN_STAGED = (size_t)4 << 20, MAX_THREADS = 6;
+    static constexpr size_t BLOCK = (size_t)1 << 20, MIN_STAGED = (size_t)8 << 20, PER_THREAD = (size_t)16 << 20,
+                            MAX_THREADS = 6;
     struct Block {
         char* p = nullptr;
         cudaEvent_t done = nullptr;
