@@ -42,9 +42,13 @@ int32_t trunc_i32(double v) {  // `as i32`: truncate and saturate, NaN -> 0
 
 // Small open-addressing set of distinct f32 values (+0.0 and -0.0 are one
 // value), tracking at most `limit` members like FeatureStats (feature_analysis.rs:296-346).
+// The slot is the product's top bits: its low bits repeat the key's, which are
+// zero in every small whole number, so such columns had one chain of all their
+// values (25 ns a value; the critical path of a table that has some: 771,484 x
+// 48 with ten of them 48 ms on 16 threads, 58 on 12, now 14 to 18).
 struct DistinctFloats {
     std::vector<uint32_t> slots;  // key bits + 1 (0 = empty)
-    uint32_t mask = 0;
+    uint32_t mask = 0, shift = 0;
     size_t size = 0;
     float first = 0.0f;
     explicit DistinctFloats(size_t limit) {
@@ -52,6 +56,7 @@ struct DistinctFloats {
         while (cap < limit * 4) cap <<= 1;
         slots.assign(cap, 0);
         mask = (uint32_t)cap - 1;
+        shift = 32u - (uint32_t)std::min(32, __builtin_ctzll(cap));
     }
     static uint32_t key(float v) {
         if (v == 0.0f) v = 0.0f;
@@ -62,7 +67,7 @@ struct DistinctFloats {
     // returns true if v is new (and inserts it when `insert`)
     bool probe(float v, bool insert) {
         uint32_t k = key(v);
-        uint32_t h = (k * 0x9E3779B1u) & mask;
+        uint32_t h = (k * 0x9E3779B1u) >> shift;
         while (true) {
             uint32_t s = slots[h];
             if (s == 0) {
