@@ -1961,19 +1961,24 @@ class Trainer {
     // WIDE_MERGE_NODES expanding nodes (the merge splits each node's many row
     // segments over more threads).
     static constexpr uint32_t WIDE_MERGE_NODES = 4;
+    // Row segments of a level whose nodes have `rows` rows in all.
+    uint64_t level_segs(uint64_t rows) const {
+        return std::max<uint64_t>((rows + bd_.hist_seg_max - 1) / bd_.hist_seg_max,
+                                  std::min<uint64_t>(bd_.hist_target, rows / 1024));
+    }
     // Whether the split search merges the partials of `nodes` nodes of `rows` rows
     // in all itself. A node of many segments has too few warps a column in the search
-    // to read them, so above SCAN_SEGS a node a merge kernel goes before
-    // it. Merged in the search / apart: the 245 segments of an fp32
-    // root of 1M x 100 41 / 35 us, the 62 of a q8 root 18.8 / 18.2; a tree of
-    // 3M x 60 (366 segments a child) fp32 2.00 / 1.93 ms, leaf-wise 5.98 / 5.82;
-    // of 1M x 100 (122) 0.92 / 0.95, leaf-wise 4.77 / 4.94.
-    // 2M x 50, q16, 296 segments of one node: 44 / 30.
-    static constexpr uint64_t SCAN_SEGS = 100;
+    // to read them, so above SCAN_SEGS a node a merge kernel goes before it: the 245
+    // segments of an fp32 root of 1M x 100 41 us merged in the search, 35 apart;
+    // of trees of depth 8 with the line at 16 / 48 / 100 a node 2M x 50 q8 take
+    // 879 / 884 / 884 us, 100K x 50 fp32 370 / 371 / 367, 1M x 200 fp32 1005 /
+    // 1001 / 996. 32-bit partials of 64-bit bins (q16) are half the bytes for the
+    // merge kernel, and the line lies at SCAN_SEGS_WIDE (0 / 8 / 16 / 24 a node):
+    // 2M x 50 918 / 900 / 901 / 909 us, 100K x 100 474 / 430 / 429 / 428, 2M x 7 of
+    // depth 10 751 / 789 / 797 / 808; with 100 there 2M x 50 of depth 6 lost 3%.
+    static constexpr uint64_t SCAN_SEGS = 100, SCAN_SEGS_WIDE = 9;
     bool scan_merges(uint64_t rows, uint64_t nodes) const {
-        const uint64_t segs = std::max<uint64_t>((rows + bd_.hist_seg_max - 1) / bd_.hist_seg_max,
-                                                 std::min<uint64_t>(bd_.hist_target, rows / 1024));
-        return segs <= SCAN_SEGS * nodes;
+        return level_segs(rows) <= (qmode_ != GRAD_F32 && !hist32_ ? SCAN_SEGS_WIDE : SCAN_SEGS) * nodes;
     }
     enum class Merge { General, All, AllWide };
     void enqueue_hist(const GradRef& gr, const uint32_t* ridx, bool root, Timer& tm, uint64_t& launches,
@@ -2858,8 +2863,12 @@ class Trainer {
         const double* scale = unit_scale(o);
         launches = 0;
         hist_launches = 0;
-        // a batch's size is not known here: by segments of the largest size
-        const bool step_merge = n_ / 2 / bd_.hist_seg_max > 128;
+        // A batch's nodes are not known here: by the segments of the first, one
+        // node's, in every precision. Merged in the search / apart, ms a tree of
+        // 255 and of 31 leaves: 500K x 200 q16 (45 segments) 2.39 / 2.62, 0.915 /
+        // 0.930; 1M x 100 q16 (90) 2.05 / 2.12, 0.937 / 0.909; 1M x 50 q16 (180)
+        // 1.88 / 1.84, 0.888 / 0.805; 2M x 50 q8 (180) 2.13 / 2.04, 1.14 / 1.02.
+        const bool step_merge = level_segs(n_ / 2) > SCAN_SEGS;
         for (uint32_t k = 0; k < LW_STEPS; ++k) {
             tm.begin(PH_OTHER);
             launch_lw_replay(bd_, lw_, lp, scale, st_);
