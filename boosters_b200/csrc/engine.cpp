@@ -1973,12 +1973,14 @@ class Trainer {
     // of trees of depth 8 with the line at 16 / 48 / 100 a node 2M x 50 q8 take
     // 879 / 884 / 884 us, 100K x 50 fp32 370 / 371 / 367, 1M x 200 fp32 1005 /
     // 1001 / 996. 32-bit partials of 64-bit bins (q16) are half the bytes for the
-    // merge kernel, and the line lies at SCAN_SEGS_WIDE (0 / 8 / 16 / 24 a node):
-    // 2M x 50 918 / 900 / 901 / 909 us, 100K x 100 474 / 430 / 429 / 428, 2M x 7 of
-    // depth 10 751 / 789 / 797 / 808; with 100 there 2M x 50 of depth 6 lost 3%.
-    static constexpr uint64_t SCAN_SEGS = 100, SCAN_SEGS_WIDE = 9;
+    // merge kernel, and the line lies at 16, for few columns, which leave it few
+    // blocks' worth of bytes, at 9 (0 / 8 / 16 / 24 a node: 2M x 50 918 / 900 /
+    // 901 / 909 us, 100K x 100 of depth 4 207 / 206 / 202 / 200; 2M x 12 670 / 672
+    // / 682 / 690, 2M x 7 of depth 10 751 / 789 / 797 / 808).
+    static constexpr uint64_t SCAN_SEGS = 100;
     bool scan_merges(uint64_t rows, uint64_t nodes) const {
-        return level_segs(rows) <= (qmode_ != GRAD_F32 && !hist32_ ? SCAN_SEGS_WIDE : SCAN_SEGS) * nodes;
+        const uint64_t line = qmode_ == GRAD_F32 || hist32_ ? SCAN_SEGS : n_cols_ < 32 ? 9 : 16;
+        return level_segs(rows) <= line * nodes;
     }
     enum class Merge { General, All, AllWide };
     void enqueue_hist(const GradRef& gr, const uint32_t* ridx, bool root, Timer& tm, uint64_t& launches,
@@ -2865,10 +2867,12 @@ class Trainer {
         hist_launches = 0;
         // A batch's nodes are not known here: by the segments of the first, one
         // node's, in every precision. Merged in the search / apart, ms a tree of
-        // 255 and of 31 leaves: 500K x 200 q16 (45 segments) 2.39 / 2.62, 0.915 /
-        // 0.930; 1M x 100 q16 (90) 2.05 / 2.12, 0.937 / 0.909; 1M x 50 q16 (180)
-        // 1.88 / 1.84, 0.888 / 0.805; 2M x 50 q8 (180) 2.13 / 2.04, 1.14 / 1.02.
-        const bool step_merge = level_segs(n_ / 2) > SCAN_SEGS;
+        // 255 and of 31 leaves: 500K x 200 q16 (84 segments) 2.36 / 2.59, 0.90 /
+        // 0.92; 1M x 100 q16 (148) 2.02 / 2.09, 0.93 / 0.90; 500K x 50 q16 (244)
+        // 1.61 / 1.64, 0.72 / 0.67; 1M x 50 q16 (296) 1.85 / 1.82, 0.89 / 0.80; 2M
+        // x 50 q8 (296) 2.09 / 2.03, 1.12 / 1.01; fp32 1M x 100 (123) 2.33 / 2.39,
+        // 1.12 / 1.09, 1M x 50 (148) 2.00 / 1.98, 0.95 / 0.88.
+        const bool step_merge = level_segs(n_ / 2) > (qmode_ == GRAD_F32 ? 128u : 200u);
         for (uint32_t k = 0; k < LW_STEPS; ++k) {
             tm.begin(PH_OTHER);
             launch_lw_replay(bd_, lw_, lp, scale, st_);
