@@ -1523,16 +1523,6 @@ class Trainer {
     }
 
     // ---- small training sets: one cooperative launch per tree (small_tree.cuh) --
-    // us per tree, one launch / level kernels (depth 6 unless said):
-    // 5,000 x 100 fp32 119 / 237; 20,000 x 100 157 / 247; 50,000 x 100 fp32
-    // 230 / 266, q8 194 / 237, depth 8 fp32 374 / 382; 52,000 x 148 234 / 278;
-    // 100,000 x 100 fp32 354 / 279, q8 278 / 259. Few columns leave most blocks
-    // without a row loop while the level kernels get cheaper: 50,000 x 40,
-    // depth 8, 354 / 324; 66,000 x 12, depth 7, 323 / 254. Several columns a
-    // block read the rows again for each: 10,000 x 300, depth 8, 486 / 483;
-    // 25,000 x 200 288 / 279; 20,000 x 300 q8, depth 8, 510 / 407. The lines lie
-    // where the level kernels cross.
-    static constexpr uint64_t SMALL_TREE_ROWS = 28000, SMALL_TREE_ROWS_F32 = 52000, SMALL_TREE_ROWS_Q = 70000;
     bool use_small_ = false;
     DevArray<uint8_t> small_buf_;  // zeroed scratch, then BState and the tree
     DevArray<uint16_t> small_rt_;
@@ -1540,6 +1530,44 @@ class Trainer {
     DevArray<longlong2> small_fix_;  // f32 form: the round's gradients in fixed point
     size_t small_zero_ = 0, small_out_ = 0, small_out_bytes_ = 0;
     SmallTree small_{};
+
+    // Rows up to which one launch a tree is the faster route. A block reads
+    // every row once per level and column of its own, while a level of the level
+    // kernels costs much the same whatever its rows, so the lines fall with the
+    // depth (a deep level's nodes pass its shared memory several times), with a
+    // second column a block, and with the columns (few leave most blocks without
+    // a row loop, and cheap level kernels); 32-bit counters (quantised forms) read
+    // less. ROWS: thousand rows at 12 and at one column per SM, by depth (<= 4,
+    // 5-6, 7, 8). Where the routes cross, measured, thousand rows at 12 / 40 / 73 /
+    // 100 / 148 columns: fp32 depth 4 49 / 62 / 68 / 68 / 82, 6 41 / 48 / 52 / 57 /
+    // 66, 7 29 / 37 / 38 / 48 / 56, 8 18 / 23 / 28 / 34 / 49; q8 79 / 94 / 99 / - / -,
+    // 63 / 70 / 72 / 81 / 106, 52 / 58 / 63 / 71 / 92, 35 / 37 / 42 / 48 / 72. Depth 6 at
+    // 149 / 200 / 296 / 297 columns: fp32 16 / 18 / 26 / 8, q8 22 / 23 / 32 / 7. With
+    // categorical columns (12, 40, 100 columns) depth 6: fp32 31 / 41 / 50, q8 50 /
+    // 64 / 67; 7: 18 / 29 / 37, 34 / 41 / 50; 8: 13 / 14 / 25, 15 / 14 / 28 (64 categories: a
+    // warp orders a node's; with 32 the lines hardly fall, with 220 they lie near 9
+    // and one launch takes up to twice as long from 20 on). At twice
+    // the crossing's rows one launch takes 1.4 to 2.3 times as long, at half 0.6 to 0.8.
+    // q16 gains most (66 at any columns up to depth 6, 60 at 12 and depth 7, 40 /
+    // 44 / 53 / 66 at depth 8; 29 / 31 / 46 / 14 for 149 to 297 columns) up to 65,536
+    // rows, where its counters become 64-bit ones (73 columns, depth 7: 0.95 ->
+    // 1.3 times the level kernels' time; there the line lies just above).
+    uint64_t small_tree_rows(uint32_t cats) const {
+        static constexpr uint32_t ROWS[3][4][2] = {{{49, 82}, {40, 66}, {28, 54}, {18, 44}},  // fp32
+                                                   {{65, 80}, {66, 66}, {56, 77}, {38, 66}},  // q16
+                                                   {{78, 112}, {60, 86}, {52, 82}, {32, 56}}};  // q8
+        const uint64_t per_block = (n_cols_ + sm_count() - 1) / sm_count();
+        const int d = cfg_.max_depth <= 4 ? 0 : cfg_.max_depth <= 6 ? 1 : (int)cfg_.max_depth - 5;
+        const int q = qmode_ == GRAD_F32 || (qmode_ == GRAD_Q8 && per_block > 1) ? 0 : qmode_ == GRAD_Q16 ? 1 : 2;
+        const double full = std::max<double>(sm_count(), 13.0), at = (double)n_cols_ / (double)per_block;
+        const double f = std::max(0.0, std::min(1.0, (at - 12.0) / (full - 12.0)));
+        double rows = 1000.0 * (ROWS[q][d][0] + f * ((double)ROWS[q][d][1] - ROWS[q][d][0])) + 100.0;
+        static constexpr double WIDE[4] = {1e9, 65536.0, 66100.0, 65536.0};  // q16
+        static constexpr double CAT[3][4] = {{0.85, 0.8, 0.65, 0.65}, {1.0, 0.9, 0.65, 0.42}, {0.85, 0.8, 0.65, 0.42}};
+        if (cats > 32) rows *= CAT[q][d] * std::min(1.0, 64.0 / cats);
+        if (per_block > 1) rows *= (q == 1 ? 1.5 : 1.15) / (double)(per_block * per_block);
+        return (uint64_t)(q == 1 ? std::min(rows, WIDE[d]) : rows);
+    }
 
     // Depth-wise batched trees of up to SMALL_TREE_DEPTH levels, without leaf
     // renewing (it needs the rows grouped by leaf), per-phase timers (they
@@ -1550,19 +1578,15 @@ class Trainer {
             cfg_.max_depth > SMALL_TREE_DEPTH || cfg_.phase_timings || cfg_.autotune_cache ||
             cfg_.objective == BST_OBJ_ABSOLUTE || cfg_.objective == BST_OBJ_PINBALL)
             return false;
-        // a block reads every row once per level and column of its own
-        const uint64_t per_block = (n_cols_ + sm_count() - 1) / sm_count();
-        const uint64_t rows = per_block > 1 || n_cols_ < sm_count() / 2 ? SMALL_TREE_ROWS
-                              : qmode_ == GRAD_F32                        ? SMALL_TREE_ROWS_F32
-                                                                          : SMALL_TREE_ROWS_Q;
-        if (n_ * per_block > rows) return false;
         uint32_t max_bins = 1;
         bool cat = false;
+        uint32_t cats = 0;  // of a categorical column, at most
         for (uint32_t c = 0; c < n_cols_; ++c) {
             max_bins = std::max(max_bins, p_.col_nbins[c]);
             cat = cat || p_.col_cat[c];
+            if (p_.col_cat[c]) cats = std::max(cats, p_.col_nbins[c]);
         }
-        return small_tree_fits(qmode_, n_, max_bins, cat);
+        return n_ <= small_tree_rows(cats) && small_tree_fits(qmode_, n_, max_bins, cat);
     }
 
     void setup_small() {

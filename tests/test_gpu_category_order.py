@@ -18,7 +18,7 @@ COUNTS = [2, 4, 5, 31, 32, 33, 63, 64, 65, 128, 129, 192, 255, 256]
 @pytest.mark.parametrize("form", ["host", "levels", "one launch"])
 @pytest.mark.parametrize("k", COUNTS)
 def test_order(form, k):
-    n = k * max(20, (30_000 if form == "levels" else 4_000) // k + 1)
+    n = k * max(20, (60_000 if form == "levels" else 4_000) // k + 1)
     rng = np.random.default_rng(k)
     cat = np.arange(n) % k
     step = rng.permutation(k)[: k // 2 + 1].astype(np.float32)
