@@ -881,8 +881,9 @@ struct RoundForest {
 
 class Trainer {
   public:
+    // speculate: batched leaf-wise growth gets slots for speculative expansions
     Trainer(const HostDataset& ds, const DeviceBinned& b, const bst_config& cfg, uint32_t n_threads,
-            cudaStream_t st, Model& model)
+            cudaStream_t st, Model& model, bool speculate)
         : ds_(ds), b_(b), p_(b.plan), cfg_(cfg), st_(st), m_(model) {
         n_ = p_.n;
         G_ = model.n_groups;
@@ -898,7 +899,7 @@ class Trainer {
         leafwise_ = cfg.growth_strategy == BST_GROWTH_LEAFWISE;
         const uint32_t max_leaves = leafwise_ ? cfg.max_leaves : (1u << std::min<uint32_t>(cfg.max_depth, 31));
         // batched leaf-wise: room for speculative expansions (grow_leafwise)
-        max_pnodes_ = std::max<uint32_t>(1, leafwise_ && cfg.batched ? 2 * max_leaves : max_leaves);
+        max_pnodes_ = std::max<uint32_t>(1, leafwise_ && cfg.batched && speculate ? 2 * max_leaves : max_leaves);
         timer_.st = st;
         timer_.enabled = cfg.phase_timings != 0;
         gp_.lambda = (double)cfg.lambda;
@@ -1452,7 +1453,8 @@ class Trainer {
             // one histogram per partition node (the reference's LRU pool is
             // unnecessary with 180 GB of HBM); refuse sizes that cannot fit
             // (the free memory is asked for only when they take a fair share
-            // of the device: the query takes 0.02 to 80 ms on a shared host)
+            // of the device: the query takes 0.02 to 80 ms on a shared host;
+            // smaller ones that do not fit after all: with_less_memory)
             double need = (double)max_pnodes_ * (double)slot_bins_ * sizeof(HBin);
             size_t free_b = std::numeric_limits<size_t>::max(), total_b = 0;
             if (need > HIST_QUERY_BYTES) BST_CK(cudaMemGetInfo(&free_b, &total_b));
@@ -3380,42 +3382,59 @@ void make_binned(const HostDataset& ds, const bst_config& cfg, cudaStream_t st, 
     out.binning_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// f(true), or f(false), which does without the speculative slots, where
+// leaf-wise growth ran out of device memory with them.
+template <class F>
+static auto with_less_memory(const bst_config& cfg, F f) {
+    try {
+        return f(true);
+    } catch (const Error& e) {
+        if (e.code != BST_ERR_OUT_OF_MEMORY || cfg.growth_strategy != BST_GROWTH_LEAFWISE || !cfg.batched) throw;
+    }
+    return f(false);
+}
+
 std::unique_ptr<Model> grow_one_tree(const HostDataset& ds, const float* g, const float* h, const bst_config& cfg,
                                      uint32_t n_threads) {
     BST_CK(cudaSetDevice(cfg.device));
     StreamGuard sg;
-    auto model = std::make_unique<Model>();
-    model->device = cfg.device;
-    model->objective = BST_OBJ_SQUARED;
-    model->n_groups = 1;
-    model->n_features = (uint32_t)ds.F;
-    model->base = {0.0f};
     DeviceBinned binned;
     make_binned(ds, cfg, sg.s, binned);
-    Trainer tr(ds, binned, cfg, n_threads, sg.s, *model);
-    HostTree t = tr.run_external(g, h);
-    model->trees.push_back(std::move(t));
-    return model;
+    return with_less_memory(cfg, [&](bool speculate) {
+        auto model = std::make_unique<Model>();
+        model->device = cfg.device;
+        model->objective = BST_OBJ_SQUARED;
+        model->n_groups = 1;
+        model->n_features = (uint32_t)ds.F;
+        model->base = {0.0f};
+        Trainer tr(ds, binned, cfg, n_threads, sg.s, *model, speculate);
+        HostTree t = tr.run_external(g, h);
+        model->trees.push_back(std::move(t));
+        return model;
+    });
 }
 
 std::unique_ptr<Model> train_model(const HostDataset& ds, const bst_config& cfg, uint32_t n_threads,
                                    const HostDataset* val) {
     BST_CK(cudaSetDevice(cfg.device));
     StreamGuard sg;
-    auto model = std::make_unique<Model>();
-    model->device = cfg.device;
-    model->objective = cfg.objective;
-    model->n_groups = n_outputs_of(cfg);
-    model->n_features = (uint32_t)ds.F;
     DeviceBinned binned;
     make_binned(ds, cfg, sg.s, binned);
-    model->timings[PH_BIN] = binned.binning_ms;
-    base_scores(ds, cfg, model->n_groups, model->base);
-    const auto t0 = std::chrono::steady_clock::now();
-    Trainer tr(ds, binned, cfg, n_threads, sg.s, *model);
-    tr.run(val);
-    model->timings[7] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    return model;
+    return with_less_memory(cfg, [&](bool speculate) {
+        auto model = std::make_unique<Model>();
+        model->device = cfg.device;
+        model->objective = cfg.objective;
+        model->n_groups = n_outputs_of(cfg);
+        model->n_features = (uint32_t)ds.F;
+        model->timings[PH_BIN] = binned.binning_ms;
+        base_scores(ds, cfg, model->n_groups, model->base);
+        const auto t0 = std::chrono::steady_clock::now();
+        Trainer tr(ds, binned, cfg, n_threads, sg.s, *model, speculate);
+        tr.run(val);
+        model->timings[7] =
+            std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        return model;
+    });
 }
 
 struct Booster::Impl {
@@ -3447,8 +3466,11 @@ Booster::Booster(const HostDataset& ds, const bst_config& cfg, uint32_t n_thread
     make_binned(ds, cfg, b.sg.s, b.binned);
     m.timings[PH_BIN] = b.binned.binning_ms;
     base_scores(ds, cfg, m.n_groups, m.base);
-    b.tr = std::make_unique<Trainer>(ds, b.binned, b.cfg, n_threads, b.sg.s, m);
-    b.tr->start();
+    with_less_memory(b.cfg, [&](bool speculate) {
+        b.tr.reset();
+        b.tr = std::make_unique<Trainer>(ds, b.binned, b.cfg, n_threads, b.sg.s, m, speculate);
+        b.tr->start();
+    });
 }
 
 Booster::~Booster() = default;
