@@ -3757,11 +3757,21 @@ void forest_predict_rows(const DeviceForest& f, const float* x, uint64_t n, uint
         launch_predict_heap(f.heap, x, n, (uint32_t)F, feature_major ? 1 : 0, out, scratch, scratch_bytes, st);
         return;
     }
-    const size_t need = std::max<size_t>(predict_heap_scratch(f.heap, (uint32_t)F, n), 16);
-    void* tmp = nullptr;
-    BST_CK(cudaMallocFromPoolAsync(&tmp, need, scratch_pool(), st));
-    launch_predict_heap(f.heap, x, n, (uint32_t)F, feature_major ? 1 : 0, out, tmp, need, st);
-    BST_CK(cudaFreeAsync(tmp, st));
+    // short of memory: the bin tiles alone, without the split trees' leaf
+    // values; then the node list, which needs none
+    for (size_t need : {predict_heap_scratch(f.heap, (uint32_t)F, n), predict_heap_scratch_min(f.heap, (uint32_t)F, n)}) {
+        void* tmp = nullptr;
+        const cudaError_t alloc = cudaMallocFromPoolAsync(&tmp, std::max<size_t>(need, 16), scratch_pool(), st);
+        if (alloc == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            continue;
+        }
+        BST_CK(alloc);
+        launch_predict_heap(f.heap, x, n, (uint32_t)F, feature_major ? 1 : 0, out, tmp, need, st);
+        BST_CK(cudaFreeAsync(tmp, st));
+        return;
+    }
+    launch_predict(f.view, x, n, (uint32_t)F, feature_major ? 1 : 0, out, st);
 }
 
 void predict_device(const Model& m, const float* x, uint64_t n, uint64_t F, bool raw, float* out, cudaStream_t st) {
