@@ -37,6 +37,7 @@ enum CheckSite : uint32_t {
     CHECK_LEAF_ROW = 4,    // leaf update row id >= rows
     CHECK_HIST_ROW = 5,    // histogram gather row id >= rows (tensor-map gather)
     CHECK_PREDICT_NODE = 6,  // traversal node link >= forest nodes
+    CHECK_SMALL_NODE = 7,    // one launch a tree: a row's node or expansion past the tree's
 };
 struct CheckRecord {
     unsigned long long violations, site, index, bound;

@@ -297,7 +297,7 @@ __device__ void st_histograms(const SmallTree& a, StShared& s, unsigned char* dy
 #pragma unroll
                 for (uint32_t u = 0; u < V; ++u) {
                     uint32_t j = t2[u];
-                    if (!root && j != ST_NONE) j = s.map[j];
+                    if (!root && j != ST_NONE) j = BST_IN(j, ST_NODES, CHECK_SMALL_NODE) ? s.map[j] : ST_NONE;
                     j1[u] = j - j0;  // rows of other passes and ST_NONE: past mm
                 }
 #pragma unroll
@@ -637,8 +637,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_small_tree(const __grid_const
         // this block's rows move to the children
         for (uint32_t i = r_begin + tid; i < r_end; i += ST_THREADS) {
             const uint32_t t = d ? a.rt[i] : 0u;  // written by this thread's block alone
+            if (!BST_IN(t, n_tn, CHECK_SMALL_NODE)) continue;
             const uint32_t jx = s.map[t];
-            if (jx == ST_NONE) continue;
+            if (jx == ST_NONE || !BST_IN(jx, n_exp, CHECK_SMALL_NODE)) continue;
             const PartWork& pw = s.work[jx];
             const uint32_t bin = pw.matrix == 0 ? (uint32_t)a.fm8[(size_t)pw.pos * a.n + i]
                                                 : (uint32_t)a.fm16[(size_t)pw.pos * a.n + i];
@@ -689,6 +690,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_small_tree(const __grid_const
     const bool moved = n_tn > 1;
     for (uint32_t i = r_begin + tid; i < r_end; i += ST_THREADS) {
         const uint32_t t = moved ? a.rt[i] : 0u;
+        if (!BST_IN(t, n_tn, CHECK_SMALL_NODE)) continue;
         long long g, h;
         if constexpr (MODE == GRAD_F32) {
             load.conv(load.raw(i), g, h);
@@ -723,6 +725,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_small_tree(const __grid_const
     __syncthreads();
     for (uint32_t i = r_begin + tid; i < r_end; i += ST_THREADS) {  // grower.rs:208-219
         const uint32_t t = moved ? a.rt[i] : 0u;
+        if (!BST_IN(t, n_tn, CHECK_SMALL_NODE)) continue;
         a.pred[i] = a.pred[i] + val[t];
         if (a.row_leaf) a.row_leaf[i] = t;
     }

@@ -594,7 +594,8 @@ bst_status bst_metric_ex(int32_t metric, const float* preds, uint32_t n_groups, 
  * BST_ERR_CHECK when its kernels recorded a violation. This reads and clears
  * the record of `device`: the number of violations and the first one's site
  * (1 partition chunk, 2 partition scatter, 3 leaf chunk, 4 leaf-update row,
- * 5 histogram-gather row, 6 traversal node), index and bound. The normal
+ * 5 histogram-gather row, 6 traversal node, 7 node of a tree grown in one
+ * launch), index and bound. The normal
  * library returns BST_ERR_UNSUPPORTED. */
 bst_status bst_check_report(int32_t device, uint64_t* violations, uint32_t* site, uint64_t* index,
                             uint64_t* bound);
