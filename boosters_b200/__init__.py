@@ -241,11 +241,14 @@ _PRECISION = {"fp32": _n.PRECISION_FP32, "q16": _n.PRECISION_Q16, "q8": _n.PRECI
 class GBDTConfig:
     """GBDT configuration with the reference's names and defaults
     (packages/boosters-python/src/config.rs:160-560, model/gbdt/config.rs:111-226),
-    plus GPU options: precision ("fp32", "q16", "q8"), batched (depth-wise
-    trees grown by a device-side level loop replayed as one CUDA graph per
-    tree; False selects the host-driven loop), cuda_graph, device, autotune
-    (time launch-shape candidates on the first trees) and autotune_cache (a
-    file keeping the chosen shapes across runs)."""
+    plus GPU options: precision ("fp32", "q16", "q8"), batched (trees grown on
+    the device, small training sets in one launch a tree, others level by level;
+    False selects the host-driven loop), cuda_graph (the level kernels of a tree
+    launched as one captured CUDA graph instead of one by one), device, autotune
+    (time launch shapes of the level kernels on the first trees) and
+    autotune_cache (a file keeping the chosen shapes across runs). A small
+    training set with autotune_cache or phase_timings takes the level kernels
+    too, which these two are about."""
 
     def __init__(self, n_estimators=100, learning_rate=0.3, objective=None, metric=None,
                  growth_strategy=GrowthStrategy.Depthwise, max_depth=6, n_leaves=31,

@@ -48,8 +48,8 @@ void dev_cache_trim();  // frees every cached block
 // for the device to be idle, as cudaFreeHost does, then keeps the block).
 void* pinned_alloc(size_t bytes);
 void pinned_free(void* p);
-void pinned_cache_trim();
-void stream_pool_trim();  // frees every cached pinned block
+void pinned_cache_trim();  // frees every cached pinned block
+void stream_pool_trim();   // destroys the idle streams kept for the next call
 
 template <class T>
 struct DevArray {
@@ -126,8 +126,9 @@ struct DeviceForest {
     HeapForest heap{};
 };
 // out [n_groups][n] raw margins of sample-major rows x [n][F] (device;
-// feature_major: x [F][n]). The shared-memory traversal bins the rows into scratch first: the caller's
-// (scratch_bytes >= what n rows need) or stream-ordered pool memory.
+// feature_major: x [F][n]). The shared-memory traversal bins the rows into
+// scratch first: the caller's (scratch_bytes >= what n rows need) or
+// stream-ordered pool memory; without either the node list is walked.
 void forest_predict_rows(const DeviceForest& f, const float* x, uint64_t n, uint64_t F, float* out, cudaStream_t st,
                          void* scratch = nullptr, size_t scratch_bytes = 0, bool feature_major = false);
 bool forest_uses_heap(const DeviceForest& f, uint64_t n, uint64_t F);

@@ -5514,7 +5514,8 @@ void launch_transform(int transform, float* out, uint32_t G, uint64_t n, cudaStr
 // One boosting round's evaluation in one pass over the rows: the new trees'
 // leaves added to the margins (trees of f, or none), the transform, and the
 // metric's per-row terms, summed in f64 into partial[block][output][2] (sum of
-// weighted terms, sum of weights) in an order that depends on n alone. The
+// weighted terms, sum of weights) in an order that depends on n and the number
+// of SMs (up to 256 rows a block, then as many blocks as four an SM). The
 // terms are those of metric_value. Before, each round built and freed a device
 // forest, ran four kernels, read every margin back and summed on the host: 60
 // rounds with 25,000 validation rows took 66.7 ms, now 43.7 (this kernel 7 us
