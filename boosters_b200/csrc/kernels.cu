@@ -4957,7 +4957,7 @@ constexpr uint32_t PREDICT_MIN_ROWS = 128;
 constexpr uint32_t BIN_NAN = 0xFFFFu;
 constexpr uint32_t BIN_THREADS = 256;         // binning pass: 8 warps per block
 constexpr uint32_t BIN_F = 8;                 // features per block of the binning pass at most
-constexpr uint32_t BIN_TAB = 256;             // staged thresholds per feature: a search tree of 8 levels
+constexpr uint32_t BIN_TAB = 256;             // staged thresholds per feature: a search tree of 8 levels, one beside it
 
 // Launch shape of the traversal: R rows per tile, the trees of each chunk
 // split over S thread groups of R threads (S > 1 for small batches: each
@@ -5078,7 +5078,9 @@ __device__ __forceinline__ uint32_t heap_bin_block(const float* __restrict__ t, 
 // conflicts: the steps' strides are powers of two) and a 16-entry block in
 // global memory (up to eight cache lines per step): 96 us for 100,003 x 100
 // sample-major rows, now 51 us (0.98 TB/s of input and bins); 16 rows 15.9,
-// now 4.1 us; 300,000 x 100 feature-major rows 124 us.
+// now 4.1 us; 300,000 x 100 feature-major rows 124 us. Trained forests reach 256
+// thresholds a feature, the tree's 255 and one beside it: searched in global
+// memory those took 300,000 x 100 rows 250 us (229 before the staging), now 182.
 template <typename BinT, bool FM>
 __global__ void __launch_bounds__(BIN_THREADS)
 k_bin_rows(HeapForest f, const float* __restrict__ x, uint64_t n, uint32_t F, uint32_t R, uint32_t FC,
@@ -5101,7 +5103,7 @@ k_bin_rows(HeapForest f, const float* __restrict__ x, uint64_t n, uint32_t F, ui
         const uint32_t o = f.thr_off[f0 + tid], e = f.thr_off[f0 + tid + 1] - o;  // e: padded entries
         uint32_t lev = 0;
         if (!(f.feat_info[f0 + tid] >> 7)) {
-            if (e <= 240u || (e == 256u && f.thr[o + 255] != f.thr[o + 255])) {  // at most 255 thresholds
+            if (e <= 256u) {
                 lev = 1;
                 while (lev < 8u && (1u << lev) - 1u < e) ++lev;
             }
@@ -5114,7 +5116,10 @@ k_bin_rows(HeapForest f, const float* __restrict__ x, uint64_t n, uint32_t F, ui
         float v = NAN;  // never <= x
         if (!lev) {  // searched in global memory: the splitters
             if (k < HEAP_SPLITTERS) v = f.spl[(size_t)(f0 + j) * HEAP_SPLITTERS + k];
-        } else if (k && k < (1u << lev)) {
+        } else if (!k) {
+            // the largest of 256: those below it are <= x when it is
+            if (f.thr_off[f0 + j + 1] - f.thr_off[f0 + j] == 256u) v = f.thr[f.thr_off[f0 + j] + 255];
+        } else if (k < (1u << lev)) {
             const uint32_t l = 31u - (uint32_t)__clz(k);
             const uint32_t at = (2u * (k - (1u << l)) + 1u) * (1u << (lev - 1u - l)) - 1u;  // in sorted order
             const uint32_t o = f.thr_off[f0 + j];
@@ -5181,7 +5186,7 @@ k_bin_rows(HeapForest f, const float* __restrict__ x, uint64_t n, uint32_t F, ui
                         }
                     }
 #pragma unroll
-                    for (uint32_t i = 0; i < RPL; ++i) b[i] -= 1u << lev;
+                    for (uint32_t i = 0; i < RPL; ++i) b[i] += (t[0] <= v[i] ? 1u : 0u) - (1u << lev);
                 } else {
                     const uint32_t lb = info & 31u;
                     const float* sp = tab + j * BIN_TAB;
