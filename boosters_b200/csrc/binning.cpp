@@ -120,7 +120,7 @@ FeatureFacts analyze(const float* col, uint64_t n, const bst_config& cfg, bool u
     // (20.3 on 16) with a pass of its own that left off at the first value.
     constexpr uint64_t BLOCK = 2048;
     uint64_t nan = 0, nonzero = 0;
-    bool all_int = true;
+    bool all_int = all_whole(col, std::min<uint64_t>(n, 32));  // most columns' answer, for little
     for (uint64_t i0 = 0; i0 < n; i0 += BLOCK) {
         const uint64_t i1 = std::min(n, i0 + BLOCK);
 #pragma omp simd reduction(+ : nan, nonzero)
