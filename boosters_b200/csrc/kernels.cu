@@ -2752,8 +2752,8 @@ void launch_leaf_update(const LeafSeg* leaves, uint32_t n_leaves, const uint32_t
 // ============================================================================
 // Device-side depth-wise growth: the level loop of TreeGrower::grow
 // (training/gbdt/grower.rs:288-337, expansion.rs:137-196) as a fixed launch
-// sequence whose sizes live in device memory (BState), so one CUDA graph
-// replays a whole tree.
+// sequence whose sizes live in device memory (BState): the host enqueues trees
+// ahead, and with cuda_graph one captured graph replays a whole tree.
 // ============================================================================
 
 namespace {
